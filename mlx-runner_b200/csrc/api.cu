@@ -14,6 +14,7 @@
 #include "api_internal.h"
 #include "aux_kernels.cuh"
 #include "qgemm.cuh"
+#include "qgemm_exact.cuh"
 #include "qmv.cuh"
 #include "qmv_mma.cuh"
 #include "qmv_pipe.cuh"
@@ -371,6 +372,17 @@ static int gemm_tile_for(const mlxq_linear* h, int x_dtype, int64_t x_stride, co
     return qgemm_tile_tokens(gemm_layer(h), x_dtype, x_stride, x, T);
 }
 
+// Long batches whose operands may not be rounded to fp16 (anything but 4-bit layers with 16-bit activations) take the
+// full-precision GEMM where the layer qualifies, from 17 tokens on.  Not while the stream is being captured: its scratch
+// memory would become allocation nodes of the caller's graph, where the kernels of run_qmv leave plain kernel nodes.
+// MLXQ_DECODE names one of those kernels and is obeyed.
+static bool exact_gemm_for(const mlxq_linear* h, int x_dtype, int64_t x_stride, const void* x, int64_t T, cudaStream_t st) {
+    if (T < 17 || T < gemm_min_tokens() || h->bits == 0 || getenv("MLXQ_DECODE") || !qgemm_exact_takes(gemm_layer(h), x_dtype, x_stride, x, T))
+        return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
 // The layer's GEMM table, built once (device memory owned by the handle).  Returns nullptr when it cannot be kept --
 // the stream is being captured, or the allocation failed -- and the GEMM then stages the table per call as before.
 // `allow_build` is false on the path that must not allocate.
@@ -419,6 +431,18 @@ int forward_impl(mlxq_linear_t h, cudaStream_t st, const void* x, int x_dtype, i
         cudaError_t err = launch_qgemm(gemm_layer(h), c, st, &why);
         if (err != cudaSuccess) return fail(MLXQ_GPU_FAILURE, "qgemm launch: %s (%s)", cudaGetErrorString(err), why);
         return MLXQ_OK;
+    }
+    if (!peer && exact_gemm_for(h, x_dtype, x_stride, x, T, st)) {
+        GemmCall c;
+        c.x = x; c.x_dtype = x_dtype; c.x_stride = x_stride; c.y = y; c.y_dtype = y_dtype; c.y_stride = y_stride; c.T = T;
+        c.err = device_error_word(h->device);
+        if (!c.err) return fail(MLXQ_GPU_FAILURE, "no error word on device %d", h->device);
+        c.table = nullptr;
+        const char* why = "";
+        const cudaError_t err = launch_qgemm_exact(gemm_layer(h), c, st, &why);
+        if (err == cudaSuccess) return MLXQ_OK;
+        if (err != cudaErrorMemoryAllocation) return fail(MLXQ_GPU_FAILURE, "qgemm launch: %s (%s)", cudaGetErrorString(err), why);
+        // no scratch memory to be had: the kernels below need none
     }
     return run_qmv(&h, 1, st, x, x_dtype, x_stride, y, y_dtype, y_stride, T, nullptr, 0, peer);
 }

@@ -1,6 +1,7 @@
 // Interface of the tensor-core dequant-GEMM (qgemm_sm100.cu).
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -45,5 +46,11 @@ cudaError_t qgemm_build_table(const GemmLayer& L, void* table, cudaStream_t st);
 size_t qgemm_table_bytes(const GemmLayer& L);
 size_t qgemm_static_table_capacity();
 cudaError_t launch_qgemm_static(const GemmLayer& L, const GemmCall& c, cudaStream_t st, const char** why);
+
+// Shared with qgemm_exact.cu: the device's stream-ordered scratch pool (nullptr when there is none), its SM count, and
+// the tensor map of a matrix of 16-bit elements in boxes with the 128-byte swizzle.
+cudaMemPool_t gemm_scratch_pool(int device);
+int gemm_sm_count(int device);
+bool gemm_map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t outer, uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer);
 
 }  // namespace mlxq

@@ -852,6 +852,12 @@ cudaMemPool_t scratch_pool(int device) {
 
 }  // namespace
 
+cudaMemPool_t gemm_scratch_pool(int device) { return scratch_pool(device); }
+int gemm_sm_count(int device) { return sm_count(device); }
+bool gemm_map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t outer, uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer) {
+    return make_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_UINT16, base, inner, outer, row_bytes, box_inner, box_outer, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
 // Batches of more than 128 tokens take the wide tile (128 rows x 256 tokens), shorter ones the tall one (256 x 128).
 static bool use_wide(long long T) { return T > 128; }
 

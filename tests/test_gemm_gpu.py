@@ -194,3 +194,51 @@ def test_prepared_table_changes_nothing(mlxq, oracle):
     assert oracle.max_rel_err(outs[0], ref) < 1e-3
     assert np.array_equal(outs[0].view(np.uint32), outs[1].view(np.uint32))
     assert np.array_equal(outs[0].view(np.uint32), outs[2].view(np.uint32))
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
+def test_full_precision_gemm_at_its_edges(mlxq, oracle, bits):
+    # the GEMM behind batches whose operands may not be rounded to fp16: one step of K and more, all group sizes, one to
+    # several row tiles and tokens tiles of 32 / 64 / 128, K split over CTAs (K = 2048: eight segments) and not, a row
+    # bias, strided rows with NaN padding.  The bound: an activation is kept to 2^-22 (two fp16 numbers), each of up to eight
+    # tensor-core steps of a group drops what lies below 2^-25 of its sum, the rest is fp32: 2^-22 + 8 * 2^-25 < 5e-7 of
+    # the terms, which cancel by less than two -- 1e-6 normwise.
+    for gs, x_dtype, T, O, K in [(32, 0, 17, 41, 128), (64, 0, 33, 129, 2048), (128, 0, 129, 264, 1280), (64, 1, 64, 127, 640),
+                                 (32, 2, 65, 300, 1152), (128, 2, 32, 40, 2048)]:
+        if bits == 4 and x_dtype != 0 and K >= 1024:
+            x_dtype = 0                                            # (4-bit layers round 16-bit activations' weights to fp16 there)
+        fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=gs, scale_type=oracle.BF16, with_bias=True, seed=T + O + bits)
+        layer = DevLayer.from_fixture(mlxq, fx)
+        x = oracle.RNG(T + K).floats(T * K).reshape(T, K)
+        xr = as_dtype(x, x_dtype).float().cpu().numpy()
+        got = run(layer, x, T, x_dtype=x_dtype, x_stride=K + 8, y_stride=O + 3)
+        mlxq.streamStatus(None, 0)
+        if bits == 4 and x_dtype != 0:
+            bar = 5e-4                                             # K = 640: the fp16-weight GEMM's bar
+        else:
+            bar = 1e-6
+        ref = _ref(oracle, fx, xr, K, bits, gs, oracle.BF16, bias=fx.bias)
+        nrm = float(np.linalg.norm(got - ref) / np.linalg.norm(ref))
+        assert nrm < bar, f"bits {bits} gs {gs} x dtype {x_dtype} T {T} {O}x{K}: normwise {nrm}"
+
+
+def test_captured_long_batches_need_no_allocation_nodes(mlxq, oracle):
+    # a stream under capture keeps the kernels that use no scratch memory; the results agree within both paths' fp32 sums
+    O, K, T = 200, 1024, 40
+    fx = oracle.QuantFixture(O=O, K=K, bits=8, gs=64, seed=9)
+    layer = DevLayer.from_fixture(mlxq, fx)
+    xv = oracle.RNG(3).floats(T * K).reshape(T, K)
+    x = torch.from_numpy(xv).cuda()
+    y = torch.full((T, O), float("nan"), device="cuda")
+    layer.linear.encode(None, x, K, y, O, T)
+    torch.cuda.synchronize()
+    eager = y.cpu().numpy()
+    y.fill_(float("nan"))
+    layer.linear.encode(None, x[:16], K, y, O, 16)                 # (function attributes are set outside the capture)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        layer.linear.encode(torch.cuda.current_stream(), x, K, y, O, T)
+    g.replay()
+    torch.cuda.synchronize()
+    mlxq.streamStatus(None, 0)
+    assert float(np.linalg.norm(y.cpu().numpy() - eager) / np.linalg.norm(eager)) < 5e-6
