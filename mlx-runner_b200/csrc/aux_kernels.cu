@@ -1,9 +1,41 @@
 // Small kernels beside the matvec / GEMM: code unpack (the bit-exact format check), embedding-row lookup
 // and the row-list matvec.  All three walk the bit stream in 8-code chunks (BITS bytes each, byte
 // aligned for every bit width).
+//
+// The kernels of a decode step (lookup, residual + norm, activation product, token selection) take part in the chain of
+// dependent launches that the matvec kernels form: each lets the next kernel of the stream start at once -- a matvec then
+// fetches its first weights meanwhile -- and waits for the previous one before it touches activations or outputs.  What an
+// earlier kernel wrote is read through L2 (ld.cg): the L1 of a grid that started early may hold older lines.  At 4096
+// columns the step of 36 layers spends 73 + 36 + 4 such launches; without the chain each left the SMs idle on either side of
+// it (with six tokens the step took 4770 us, with the chain 4326).
 #include "aux_kernels.cuh"
 
+#include <cstdlib>
+
 namespace mlxq {
+
+namespace {
+
+__device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launches `kernel` as a programmatic dependent of the stream's previous kernel (MLXQ_PDL=0: as an ordinary one).
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+    static const bool pdl = [] { const char* e = std::getenv("MLXQ_PDL"); return !(e && e[0] == '0'); }();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cudaLaunchAttribute la[1];
+    la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    la[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = la;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+}  // namespace
 
 // out[r, k] = code k of row r, one byte each.  One thread per 8-code chunk.
 __global__ void unpack_codes_kernel(const uint8_t* __restrict__ w, uint8_t* __restrict__ out, long long rows, int K,
@@ -25,10 +57,12 @@ __global__ void unpack_codes_kernel(const uint8_t* __restrict__ w, uint8_t* __re
 __global__ void lookup_kernel(const uint8_t* __restrict__ w, const void* __restrict__ scales, const void* __restrict__ biases,
                               int s_dtype, const int32_t* __restrict__ ids, float* __restrict__ out, int rows, int K, int gs,
                               int bits, unsigned* err) {
+    if (threadIdx.x == 0) dependents_may_start();
     const int t = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= K / 8) return;
-    const int row = __ldg(ids + t);
+    wait_for_previous();
+    const int row = __ldcg(ids + t);
     float* o = out + static_cast<size_t>(t) * K + c * 8;
     if (row < 0 || row >= rows) {
         if (c == 0) atomicOr(err, ERR_BAD_LOOKUP_ID);
@@ -94,10 +128,11 @@ cudaError_t launch_lookup(const uint8_t* w, const void* scales, const void* bias
     // gridDim.y is limited to 65535: walk longer id lists in slices.
     for (long long t0 = 0; t0 < T; t0 += 65535) {
         const unsigned ty = static_cast<unsigned>(T - t0 < 65535 ? T - t0 : 65535);
-        lookup_kernel<<<dim3((chunks + block - 1) / block, ty), block, 0, st>>>(
-            w, scales, biases, s_dtype, ids + t0, out + static_cast<size_t>(t0) * K, rows, K, gs, bits, err);
+        const cudaError_t e = launch_dependent(lookup_kernel, dim3((chunks + block - 1) / block, ty), dim3(block), st, w, scales, biases, s_dtype,
+                                               ids + t0, out + static_cast<size_t>(t0) * K, rows, K, gs, bits, err);
+        if (e != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 cudaError_t launch_rows(const uint8_t* w, const void* scales, const void* biases, int s_dtype, const void* x, int x_dtype,
@@ -116,9 +151,11 @@ cudaError_t launch_rows(const uint8_t* w, const void* scales, const void* biases
 // hold it, the lowest index.  bmax[t][b] / barg[t][b]; a block without any value above -inf reports SELECT_NONE.
 __global__ void block_max_kernel(const float* __restrict__ logits, long long stride, long long V, int nb, long long T,
                                  int index_base, float* __restrict__ bmax, int* __restrict__ barg, int vec_ok) {
+    if (threadIdx.x == 0) dependents_may_start();
     const int lane = threadIdx.x & 31;
     const long long wid = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (wid >= T * nb) return;
+    wait_for_previous();
     const long long t = wid / nb;
     const int b = static_cast<int>(wid - t * nb);
     const float* row = logits + t * stride;
@@ -126,12 +163,12 @@ __global__ void block_max_kernel(const float* __restrict__ logits, long long str
     float best = -INFINITY;
     int bi = SELECT_NONE;
     if (vec_ok && i0 + 8 <= V) {
-        const float4 a = *reinterpret_cast<const float4*>(row + i0), c = *reinterpret_cast<const float4*>(row + i0 + 4);
+        const float4 a = __ldcg(reinterpret_cast<const float4*>(row + i0)), c = __ldcg(reinterpret_cast<const float4*>(row + i0 + 4));
         const float v[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
 #pragma unroll
         for (int j = 0; j < 8; j++) if (v[j] > best) { best = v[j]; bi = static_cast<int>(i0) + j; }
     } else {
-        for (long long i = i0; i < V && i < i0 + 8; i++) { const float v = row[i]; if (v > best) { best = v; bi = static_cast<int>(i); } }
+        for (long long i = i0; i < V && i < i0 + 8; i++) { const float v = __ldcg(row + i); if (v > best) { best = v; bi = static_cast<int>(i); } }
     }
     float m = best;
 #pragma unroll
@@ -151,6 +188,8 @@ __global__ void block_argmax_kernel(const uint32_t* __restrict__ pairs, int n_se
                                     float* __restrict__ value) {
     __shared__ float sm[8];
     __shared__ int si[8];
+    if (threadIdx.x == 0) dependents_may_start();
+    wait_for_previous();
     const long long t = blockIdx.x;
     const long long seg_words = 2 * T * nb;
     float best = -INFINITY;
@@ -158,8 +197,8 @@ __global__ void block_argmax_kernel(const uint32_t* __restrict__ pairs, int n_se
     for (int i = threadIdx.x; i < n_seg * nb; i += blockDim.x) {
         const int seg = i / nb, b = i - seg * nb;
         const uint32_t* base = pairs + seg * seg_words;
-        const float m = __uint_as_float(base[t * nb + b]);
-        const int ix = static_cast<int>(base[T * nb + t * nb + b]);
+        const float m = __uint_as_float(__ldcg(base + t * nb + b));
+        const int ix = static_cast<int>(__ldcg(base + T * nb + t * nb + b));
         if (m > best || (m == best && ix < bi)) { best = m; bi = ix; }
     }
     float m = best;
@@ -192,72 +231,110 @@ cudaError_t launch_block_max(const float* logits, long long stride, long long V,
     const int warps = 8;
     const long long n = T * nb;
     const int vec_ok = (reinterpret_cast<uintptr_t>(logits) % 16 == 0 && stride % 4 == 0) ? 1 : 0;
-    block_max_kernel<<<static_cast<unsigned>((n + warps - 1) / warps), warps * 32, 0, st>>>(
-        logits, stride, V, nb, T, index_base, reinterpret_cast<float*>(pairs), reinterpret_cast<int*>(pairs) + T * nb, vec_ok);
-    return cudaGetLastError();
+    return launch_dependent(block_max_kernel, dim3(static_cast<unsigned>((n + warps - 1) / warps)), dim3(warps * 32), st, logits, stride, V, nb, T,
+                            index_base, reinterpret_cast<float*>(pairs), reinterpret_cast<int*>(pairs) + T * nb, vec_ok);
 }
 
 cudaError_t launch_block_argmax(const uint32_t* pairs, int n_seg, long long T, int nb, int32_t* token, float* value, cudaStream_t st) {
     if (T == 0) return cudaSuccess;
-    block_argmax_kernel<<<static_cast<unsigned>(T), 256, 0, st>>>(pairs, n_seg, T, nb, token, value);
-    return cudaGetLastError();
+    return launch_dependent(block_argmax_kernel, dim3(static_cast<unsigned>(T)), dim3(256), st, pairs, n_seg, T, nb, token, value);
 }
 
 // ---- silu_mul / gelu_tanh_mul (Kernels.swift:2004-2030): out[t, i] = act(gu[t, i]) * gu[t, cols + i] ----------------
-__global__ void act_mul_kernel(const float* __restrict__ gu, long long stride, long long cols, int act, float* __restrict__ out) {
+// `vec`: four elements per thread (rows and columns are whole 16-byte pieces), else one.
+__global__ void act_mul_kernel(const float* __restrict__ gu, long long stride, long long cols, int act, float* __restrict__ out, int vec) {
+    if (threadIdx.x == 0) dependents_may_start();
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const long long t = blockIdx.y;
-    if (i >= cols) return;
-    const float g = gu[t * stride + i], u = gu[t * stride + cols + i];
+    if (i >= (vec ? cols / 4 : cols)) return;
+    wait_for_previous();
+    if (vec) {
+        const float4 g = __ldcg(reinterpret_cast<const float4*>(gu + t * stride) + i), u = __ldcg(reinterpret_cast<const float4*>(gu + t * stride + cols) + i);
+        reinterpret_cast<float4*>(out + t * cols)[i] = make_float4(act_mul(act, g.x, u.x), act_mul(act, g.y, u.y), act_mul(act, g.z, u.z), act_mul(act, g.w, u.w));
+        return;
+    }
+    const float g = __ldcg(gu + t * stride + i), u = __ldcg(gu + t * stride + cols + i);
     out[t * cols + i] = act_mul(act, g, u);
 }
 
 // ---- add_rms_norm (Kernels.swift:1141-1175): h += r; y = RMSNorm(h) * w, one CTA per row.  The sum of squares is
-// taken per thread over float4s in a strided order, then per warp, then over the warps in order, as the reference's
-// threadgroup does; dim is a multiple of 4 and the rows are 16-byte aligned (checked on the host). -------------------
-__global__ void add_rms_norm_kernel(float* __restrict__ hbuf, const float* __restrict__ r, float* __restrict__ y, const void* __restrict__ w,
-                                    int w_dtype, int dim, long long row_stride, float eps) {
+// taken per thread over float4s in a strided order, then per warp, then over the warps, as the reference's threadgroup
+// does; dim is a multiple of 4 and the rows are 16-byte aligned (checked on the host).  Bound by latency -- load, reduce,
+// store -- so a row gets a thread per float4 up to 1024 threads, and a thread keeps its first NORM_KEEP float4s in
+// registers between the two passes (4096 columns: one pass over memory; 3.7 -> 2.8 us a call back to back, with the
+// dependent launch). ----------------------------------------------------------------------------------------------------
+constexpr int NORM_KEEP = 4;
+__global__ void __launch_bounds__(1024) add_rms_norm_kernel(float* __restrict__ hbuf, const float* __restrict__ r, float* __restrict__ y, const void* __restrict__ w,
+                                                            int w_dtype, int dim, long long row_stride, float eps) {
     __shared__ float buf[32];
+    if (threadIdx.x == 0) dependents_may_start();
     const long long row = blockIdx.x;
     float4* hr = reinterpret_cast<float4*>(hbuf + row * row_stride);
     const float4* rr = reinterpret_cast<const float4*>(r + row * row_stride);
     float4* yr = reinterpret_cast<float4*>(y + row * row_stride);
-    const int n4 = dim / 4;
+    const int n4 = dim / 4, nt = blockDim.x;
+    wait_for_previous();
+    float4 kept[NORM_KEEP];
     float ss = 0.0f;
-    for (int i = threadIdx.x; i < n4; i += blockDim.x) {
-        const float4 a = hr[i], b = rr[i];
+#pragma unroll
+    for (int k = 0; k < NORM_KEEP; k++) {
+        const int i = threadIdx.x + k * nt;
+        if (i < n4) {
+            const float4 a = __ldcg(hr + i), b = __ldcg(rr + i);
+            kept[k] = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NORM_KEEP; k++) {
+        const int i = threadIdx.x + k * nt;
+        if (i < n4) {
+            const float4 v = kept[k];
+            hr[i] = v;
+            ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        }
+    }
+    for (int i = threadIdx.x + NORM_KEEP * nt; i < n4; i += nt) {
+        const float4 a = __ldcg(hr + i), b = __ldcg(rr + i);
         const float4 v = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
         hr[i] = v;
         ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nt >> 5;
     if (lane == 0) buf[warp] = ss;
     __syncthreads();
-    float tot = 0.0f;
-    for (int s = 0; s < nw; s++) tot += buf[s];
+    float tot = lane < nw ? buf[lane] : 0.0f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
     const float inv = rsqrtf(tot / static_cast<float>(dim) + eps);
-    for (int i = threadIdx.x; i < n4; i += blockDim.x) {
-        const float4 v = hr[i];
+    auto scaled = [&](int i, const float4 v) {
         const float w0 = load_scalar(w, w_dtype, 4 * i), w1 = load_scalar(w, w_dtype, 4 * i + 1), w2 = load_scalar(w, w_dtype, 4 * i + 2),
                     w3 = load_scalar(w, w_dtype, 4 * i + 3);
         yr[i] = make_float4(v.x * inv * w0, v.y * inv * w1, v.z * inv * w2, v.w * inv * w3);
+    };
+#pragma unroll
+    for (int k = 0; k < NORM_KEEP; k++) {
+        const int i = threadIdx.x + k * nt;
+        if (i < n4) scaled(i, kept[k]);
     }
+    for (int i = threadIdx.x + NORM_KEEP * nt; i < n4; i += nt) scaled(i, hr[i]);
 }
 
 cudaError_t launch_act_mul(const float* gu, long long stride, long long cols, long long T, int act, float* out, cudaStream_t st) {
     if (T == 0) return cudaSuccess;
     if (T > 65535) return cudaErrorInvalidValue;
-    act_mul_kernel<<<dim3(static_cast<unsigned>((cols + 255) / 256), static_cast<unsigned>(T)), 256, 0, st>>>(gu, stride, cols, act, out);
-    return cudaGetLastError();
+    const int vec = (cols % 4 == 0 && stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0) ? 1 : 0;
+    const long long n = vec ? cols / 4 : cols;
+    return launch_dependent(act_mul_kernel, dim3(static_cast<unsigned>((n + 255) / 256), static_cast<unsigned>(T)), dim3(256), st, gu, stride, cols, act, out, vec);
 }
 
 cudaError_t launch_add_rms_norm(float* h, const float* r, float* y, const void* w, int w_dtype, long long dim, long long rows,
                                 long long row_stride, float eps, cudaStream_t st) {
     if (rows == 0) return cudaSuccess;
-    add_rms_norm_kernel<<<static_cast<unsigned>(rows), 256, 0, st>>>(h, r, y, w, w_dtype, static_cast<int>(dim), row_stride, eps);
-    return cudaGetLastError();
+    const long long n4 = dim / 4;
+    const unsigned threads = static_cast<unsigned>(n4 < 1024 ? (n4 + 31) / 32 * 32 : 1024);
+    return launch_dependent(add_rms_norm_kernel, dim3(static_cast<unsigned>(rows)), dim3(threads), st, h, r, y, w, w_dtype, static_cast<int>(dim), row_stride, eps);
 }
 
 }  // namespace mlxq
