@@ -32,7 +32,7 @@ bool pdl_enabled() {
     return v;
 }
 
-template <int BITS, int NP, int UNR, int GS>
+template <int BITS, int NP, int UNR, int GS, int SPX>
 cudaError_t launch_one(const MmaParams& p, const PipePlan& pp, size_t smem, int device, cudaStream_t st) {
     // The shared-memory opt-in is an attribute of the function in one device's context: once per device, with
     // that device current (the caller has selected it).
@@ -42,7 +42,7 @@ cudaError_t launch_one(const MmaParams& p, const PipePlan& pp, size_t smem, int 
     {
         std::lock_guard<std::mutex> lk(mu);
         if (!done[device]) {
-            const cudaError_t e = cudaFuncSetAttribute(qmv_pipe_kernel<BITS, NP, UNR, GS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_WHOLE);
+            const cudaError_t e = cudaFuncSetAttribute(qmv_pipe_kernel<BITS, NP, UNR, GS, SPX>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_WHOLE);
             if (e != cudaSuccess) return e;
             done[device] = true;
         }
@@ -57,18 +57,26 @@ cudaError_t launch_one(const MmaParams& p, const PipePlan& pp, size_t smem, int 
     la[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = la;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, qmv_pipe_kernel<BITS, NP, UNR, GS>, p, pp);
+    return cudaLaunchKernelEx(&cfg, qmv_pipe_kernel<BITS, NP, UNR, GS, SPX>, p, pp);
+}
+
+template <int BITS, int UNR, int GS>
+cudaError_t launch_special(const MmaParams& p, const PipePlan& pp, size_t smem, int device, cudaStream_t st) {
+    if constexpr (MmaUnit<BITS>::KB <= 4 * GS) {
+        if (p.split == 2) return launch_one<BITS, 1, UNR, GS, 2>(p, pp, smem, device, st);
+    }
+    return launch_one<BITS, 1, UNR, GS, 1>(p, pp, smem, device, st);
 }
 
 template <int BITS, int UNR>
 cudaError_t launch_np(const MmaParams& p, const PipePlan& pp, size_t smem, int device, cudaStream_t st) {
     // the one-token kernels with the column plan folded in at compile time
-    if (pp.special == 32) return launch_one<BITS, 1, UNR, 32>(p, pp, smem, device, st);
-    if (pp.special == 64) return launch_one<BITS, 1, UNR, 64>(p, pp, smem, device, st);
-    if (pp.special == 128) return launch_one<BITS, 1, UNR, 128>(p, pp, smem, device, st);
-    if (p.passes <= 1) return launch_one<BITS, 1, UNR, 0>(p, pp, smem, device, st);
-    if (p.passes <= 2) return launch_one<BITS, 2, UNR, 0>(p, pp, smem, device, st);
-    if (p.passes <= 4) return launch_one<BITS, 4, UNR, 0>(p, pp, smem, device, st);
+    if (pp.special == 32) return launch_special<BITS, UNR, 32>(p, pp, smem, device, st);
+    if (pp.special == 64) return launch_special<BITS, UNR, 64>(p, pp, smem, device, st);
+    if (pp.special == 128) return launch_special<BITS, UNR, 128>(p, pp, smem, device, st);
+    if (p.passes <= 1) return launch_one<BITS, 1, UNR, 0, 1>(p, pp, smem, device, st);
+    if (p.passes <= 2) return launch_one<BITS, 2, UNR, 0, 1>(p, pp, smem, device, st);
+    if (p.passes <= 4) return launch_one<BITS, 4, UNR, 0, 1>(p, pp, smem, device, st);
     return cudaErrorNotSupported;
 }
 
@@ -150,17 +158,20 @@ size_t qmv_pipe_plan(int bits, const MmaParams& p, int tokens, int sms, PipePlan
             const int g0 = (c0 >> 8) & 255, g1 = (c1 >> 8) & 255;
             pairs = pairs && (c0 & 255) == (c1 & 255) && g1 == g0 + 1 && (g0 & 1) == 0 && g0 == static_cast<int>((f0 >> 8) & 255);
         }
+    // (the one-token kernel for fp32 activations has a column plan of its own in which they always are)
+    const bool two_parts = tokens == 1 && p.split == 2 && p.xn == 2 && kb <= 4 * q.gs && dtype_size(q.s_dtype) == 2 && groups % 2 == 0;
     pp.async_sb = pairs ? 1 : 0;
     // (the one-token kernels assume slices of whole drain cycles)
     bool whole_cycles = true;
     {
-        const int spc = p.cycle << p.spg_shift;
+        const int gsh = p.gstep_shift, cycle = two_parts ? 4 >> gsh : p.cycle, spc = cycle << p.spg_shift;
         for (int kw = 0; kw < pp.ks; kw++) {
             const int a = ((nblk * kw) >> pp.ks_shift) << p.spg_shift, b = ((nblk * (kw + 1)) >> pp.ks_shift) << p.spg_shift;
             if (a % spc != 0 || b % spc != 0) whole_cycles = false;
         }
     }
-    pp.special = (whole_cycles && tokens == 1 && p.split == 1 && p.xn == 1 && pp.async_sb && pp.rowsum && (q.gs == 32 || q.gs == 64 || q.gs == 128)) ? q.gs : 0;
+    const bool one_part = tokens == 1 && p.split == 1 && p.xn == 1 && pp.async_sb;
+    pp.special = (whole_cycles && (one_part || two_parts) && pp.rowsum && (q.gs == 32 || q.gs == 64 || q.gs == 128)) ? q.gs : 0;
     int off = align_up(p.xn * pp.xstride * 2, 16);
     pp.off_xsum = off; off += align_up(p.xn * groups * 4, 16);
     pp.off_zero = off; off += PIPE_ZERO_BYTES;
@@ -176,6 +187,7 @@ size_t qmv_pipe_plan(int bits, const MmaParams& p, int tokens, int sms, PipePlan
     }
     pp.depth = PIPE_DEPTH;
     long long total = static_cast<long long>(pp.off_ring) + static_cast<long long>(warps) * pp.depth * slot_bytes;
+    if (total > SMEM_WHOLE && two_parts) pp.special = 0;        // (the one-token kernels have the full ring only)
     if (total > SMEM_WHOLE && !pp.special) {
         pp.depth = 2;
         total = static_cast<long long>(pp.off_ring) + static_cast<long long>(warps) * pp.depth * slot_bytes;

@@ -44,7 +44,8 @@ struct PipePlan {
     int off_part;        // partial sums [groups of warps][2][ks][16 * tokens] floats
     int off_ring;        // per warp: depth slots of 2 x 32 lanes x lane bytes, then 4 x 32 x 4 bytes of (scale, bias) pairs
     int rowsum;          // 1: one token in one accumulator set -- partials come from two shuffles instead of the tile
-    int special;         // 32 / 64 / 128: the one-token kernel compiled for that group size serves the call; 0: the general one
+    int special;         // 32 / 64 / 128: the one-token kernel compiled for that group size serves the call (16-bit activations
+                         // with p.split == 1, fp32 ones with p.split == 2); 0: the general one
     int async_sb;        // 1: the drains' (scale, bias) pairs travel through the ring (see pipe_col_pairs)
     // What accumulator column n of pass ps stands for (the column plan of qmv_mma.cuh, worked out once on the host):
     // bits 0-7 staged activation column (255: none), 8-15 group offset inside the cycle block, 16-19 cycle position,
@@ -230,8 +231,12 @@ constexpr int pipe_log2(int v) { int s = 0; while ((1 << s) < v) s++; return s; 
 // GS = 0: any call, the column plan is read from the launch parameters.  GS = 32, 64, 128: the one-token call with
 // 16-bit activations and 16-bit scales at that group size -- the plan is then known at compile time (one pass, a
 // drain cycle of eight consecutive groups, the lane's two accumulator columns are groups 2t and 2t + 1 of it, the
-// pairs travel through the ring), and most of the bookkeeping below folds away.
-template <int BITS, int NP, int UNR, int GS>
+// pairs travel through the ring), and most of the bookkeeping below folds away.  SPX = 2: the same for fp32 activations,
+// whose two fp16 parts take four accumulator columns each -- columns 0-3 the high parts of four consecutive groups, 4-7 the
+// low parts -- so that a lane's two columns are again consecutive groups of one part and a drain closes every four groups.
+// (On the general plan 24576 rows of 4096 4-bit codes took 22.4 us, here 19.8; 8-bit 31.4 -> 23.9; a bf16 token 14.7 / 20.1.
+// A 151936 x 4096 head at 6 bits: 139 -> 117 us.)
+template <int BITS, int NP, int UNR, int GS, int SPX>
 __global__ void __launch_bounds__(PIPE_WARPS * 32, 1)
 qmv_pipe_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ PipePlan pp) {
     using U = MmaUnit<BITS>;
@@ -240,7 +245,8 @@ qmv_pipe_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ Pip
     static_assert(!SP || NP == 1, "the one-token plan has one pass");
     constexpr int SP_GSH = !SP ? 0 : (KB > GS ? pipe_log2(KB / GS) : 0);      // log2(groups per step)
     constexpr int SP_SPG = !SP ? 0 : (GS > KB ? pipe_log2(GS / KB) : 0);      // log2(steps per group)
-    constexpr int SP_CY = !SP ? 1 : ((8 >> SP_GSH) > 0 ? (8 >> SP_GSH) : 1);  // group blocks per drain cycle
+    constexpr int SP_CY = !SP ? 1 : (((8 / SPX) >> SP_GSH) > 0 ? ((8 / SPX) >> SP_GSH) : 1);  // group blocks per drain cycle
+    static_assert(SPX == 1 || (SP && SP_GSH <= 2), "two parts leave four columns for the groups of a step");
     // One-token plan: every slice holds whole drain cycles of SP_SPC steps (the planner sees to it) and starts on a
     // multiple of UNR, so within a loop turn only the last step can close a cycle when UNR divides SP_SPC; and both halves
     // of a step's MMAs read the same group when a lane's run does not straddle groups.
@@ -259,7 +265,7 @@ qmv_pipe_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ Pip
     const int K = q.K, gs_shift = SP ? pipe_log2(GS) : q.gs_shift;
     const int groups = K >> gs_shift;
     const int sbytes = SP ? 2 : dtype_size(q.s_dtype);
-    const int T = SP ? 1 : q.T, xn = SP ? 1 : p.xn, split = SP ? 1 : p.split;
+    const int T = SP ? 1 : q.T, xn = SP ? SPX : p.xn, split = SP ? SPX : p.split;
     const bool rowsum = SP ? true : pp.rowsum != 0;
     __half* xs = reinterpret_cast<__half*>(smem_pipe);                                   // [xn][xstride]
     float* xsum = reinterpret_cast<float*>(smem_pipe + pp.off_xsum);                     // [xn][groups]
@@ -310,16 +316,18 @@ qmv_pipe_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ Pip
 #pragma unroll
     for (int ps = 0; ps < NP; ps++) {
         const uint32_t ce = SP ? 0u : pp.col[ps][g];            // the column this lane feeds as B (column n = g)
-        const int xc = SP ? 0 : ce & 255, cyc = SP ? g >> SP_GSH : (ce >> 16) & 15, grp = SP ? g & ((1 << SP_GSH) - 1) : (ce >> 20) & 15;
-        const bool valid = SP ? (g >> SP_GSH) < SP_CY : xc != 255;
+        const int gc = SPX == 2 ? g & 3 : g;                    // the column's group inside a cycle (one-token plan)
+        const int xc = SP ? (SPX == 2 ? g >> 2 : 0) : ce & 255, cyc = SP ? gc >> SP_GSH : (ce >> 16) & 15, grp = SP ? gc & ((1 << SP_GSH) - 1) : (ce >> 20) & 15;
+        const bool valid = SP ? (gc >> SP_GSH) < SP_CY : xc != 255;
         baddr[ps] = smem_u32(xs) + ((valid ? xc : 0) * pp.xstride + t * CL) * 2;
         b_on_a[ps] = (valid && grp == run_grp_a) ? cyc : -1;
         b_on_b[ps] = (valid && grp == run_grp_b) ? cyc : -1;
 #pragma unroll
         for (int ci = 0; ci < 2; ci++) {
             const uint32_t cc = SP ? 0u : pp.col[ps][2 * t + ci];   // the lane's accumulator columns 2t, 2t + 1
-            c_xc[ps][ci] = SP ? (((2 * t + ci) >> SP_GSH) < SP_CY ? 0 : -1) : (cc & 255) == 255 ? -1 : static_cast<int>(cc & 255);
-            c_goff[ps][ci] = SP ? 2 * t + ci : (cc >> 8) & 255;
+            const int tc = SPX == 2 ? 2 * (t & 1) + ci : 2 * t + ci;
+            c_xc[ps][ci] = SP ? ((tc >> SP_GSH) < SP_CY ? (SPX == 2 ? t >> 1 : 0) : -1) : (cc & 255) == 255 ? -1 : static_cast<int>(cc & 255);
+            c_goff[ps][ci] = SP ? tc : (cc >> 8) & 255;
         }
     }
     const bool async_sb = SP ? true : pp.async_sb != 0;

@@ -180,6 +180,19 @@ def test_small_batches_every_width_and_group(mlxq, oracle, bits):
 
 
 @pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
+def test_one_fp32_token_every_width_and_group(mlxq, oracle, bits):
+    # one fp32 token: its two fp16 parts on the kernel compiled for the group size, where slices of K hold whole drain
+    # cycles of four groups, and on the general plan where they do not (K = 768); odd numbers of blocks and of steps
+    for gs in (32, 64, 128):
+        for K, O in ((768, 24), (1024, 40), (1536, 72), (5120, 17)):
+            fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=gs, scale_type=oracle.BF16 if K % 1024 else oracle.F16, with_bias=(O == 72), seed=bits + gs + K)
+            layer = DevLayer.from_fixture(mlxq, fx)
+            x = oracle.RNG(K + gs + bits).floats(K).reshape(1, K)
+            # (the split leaves 2^-22 of every product, the sums are fp32: the small batches' bar for fp32 activations)
+            close(oracle, run(layer, x, 1), fx.reference(x), f"bits {bits} gs {gs} {O}x{K}", 1e-4)
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
 def test_quantized_embedding_lookup(mlxq, oracle, bits):
     # KernelTests.swift:287-296 (4-bit there; every width here)
     K, V = 128, 16
