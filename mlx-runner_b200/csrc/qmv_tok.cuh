@@ -15,6 +15,12 @@
 // the A fragment of the bias MMA -- and hands a group's scales to the other lanes of its row by shuffle.  Everything
 // else (warp-private cp.async rings, K split over `ks` warps with a named barrier per group of warps, dependent
 // launch, the peers' stores of sharded calls) is as in qmv_pipe.cuh.
+//
+// Long rows: K is also split over the `kz` CTAs of a thread-block cluster.  Each CTA stages only its slice of the
+// activations -- with all of K a CTA's shared memory holds 8 tokens of 12288, 4 in fp32, and the call fell back to two
+// calls of half the tokens on the one-token kernel -- and multiplies that slice of the cluster's blocks; the blocks' sums
+// stay in shared memory until the end, one cluster barrier later every CTA adds up and stores a share of them, reading the
+// others' through distributed shared memory in the order of the slices.
 #pragma once
 
 #include "qmv_pipe.cuh"
@@ -24,16 +30,18 @@ namespace mlxq {
 constexpr int TOK_WARPS = 16;
 
 struct TokPlan {
-    int ks, ks_shift;    // warps that share a block along K and its log2
+    int kz, kz_shift;    // CTAs (a cluster) that share a block along K and its log2
+    int off_z;           // kz > 1: the CTA's sums [block of the cluster][token][16 rows] floats
+    int ks, ks_shift;    // warps that share a block along the CTA's slice of K and its log2
     int depth;           // ring slots (groups in flight) per warp: 8, 4 or 2
     int ntab;            // buffers of the per-block (scale, bias) cells: blocks the copy cursor may run ahead, plus two
     int nwin;            // windows of eight groups per warp slice
     int slice_groups;    // groups of the longest warp slice (slices are cut at even groups: floor(pairs * kw / ks) * 2)
     int grid, n_blocks, base_blocks, extra_blocks;
-    int cpr_shift;       // log2(in_dim / 8) when that is a power of two, else -1
+    int cpr_shift;       // log2(chunks of eight activations in the CTA's slice) when that is a power of two, else -1
     int xstride;         // halves between staged activation columns
     int tp;              // floats per row of a partial-sum tile (tokens + 1)
-    int gpad;            // floats per staged column of a part of the group sums (groups + 8, the tail zero)
+    int gpad;            // floats per staged column of a part of the group sums (the slice's groups + 8, the tail zero)
     int off_parts;       // [3][staged columns][gpad] floats: the TF32 parts of the activations' group sums
     int off_zero;        // PIPE_ZERO_BYTES of zeros (B fragments of idle columns)
     int parities;        // partial-sum slots per group of warps: 2 (alternating by block), or 1 where shared memory is short
@@ -76,6 +84,18 @@ __device__ __forceinline__ void mma1688_tf32(float (&d)[4], uint32_t a0, uint32_
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the float at shared address `addr` of CTA `rank` of the cluster
+__device__ __forceinline__ float cluster_load(uint32_t addr, int rank) {
+    uint32_t remote;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+    return v;
+}
+
 // DEPTH_CT: the ring depth when it is the width's usual one (compiled in), 0 when the planner had to take a shallower ring.
 template <int BITS, int GS, int NP, int DEPTH_CT>
 __global__ void __launch_bounds__(TOK_WARPS * 32, 1)
@@ -106,9 +126,13 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
 
     // this warp's place: group `gi` of warps in the CTA, slice `kw` of K
     const int ks = tp.ks, gi = warp >> tp.ks_shift, kw = warp & (ks - 1), n_groups = TOK_WARPS >> tp.ks_shift;
-    // the slice: quantisation groups [gmin, gmin + slice_groups), cut at even groups so that (scale, bias) pairs stay whole
-    const int gmin = (((groups >> 1) * kw) >> tp.ks_shift) << 1;
-    const int slice_groups = ((((groups >> 1) * (kw + 1)) >> tp.ks_shift) << 1) - gmin;
+    // the CTA's slice of K: groups [gb, gb + cg); the warp's: [gmin, gmin + slice_groups) of those.  Both are cut at even
+    // groups so that (scale, bias) pairs stay whole.
+    const int kz = tp.kz, rank = blockIdx.x & (kz - 1), cid = blockIdx.x >> tp.kz_shift, n_cl = gridDim.x >> tp.kz_shift;
+    const int gb = (((groups >> 1) * rank) >> tp.kz_shift) << 1;
+    const int cg = ((((groups >> 1) * (rank + 1)) >> tp.kz_shift) << 1) - gb;
+    const int gl0 = (((cg >> 1) * kw) >> tp.ks_shift) << 1, gmin = gb + gl0;
+    const int slice_groups = ((((cg >> 1) * (kw + 1)) >> tp.ks_shift) << 1) - gl0;
     // A group's bytes of the warp's sixteen rows lie row after row in a slot (RB bytes each); the warp copies them as
     // 16-byte pieces, lane l the pieces l, l + 32, ... below NPIECE, so that the copies read whole sectors whatever
     // the width; a lane then consumes GB bytes at GB * t of rows g and g + 8, which other lanes may have copied.
@@ -138,11 +162,11 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
     };
 
     // ---- the copy stream: this warp's (block, group) pairs in order, `depth` groups in flight -------------------
-    const int cta_blocks = tp.base_blocks + (static_cast<int>(blockIdx.x) < tp.extra_blocks ? 1 : 0);
+    const int cta_blocks = tp.base_blocks + (cid < tp.extra_blocks ? 1 : 0);
     const int my_blocks = cta_blocks > gi ? (cta_blocks - 1 - gi) / n_groups + 1 : 0;
-    const int blk_stride = n_groups * gridDim.x;
+    const int blk_stride = n_groups * n_cl;
     int l_left = my_blocks * slice_groups;                     // groups not yet issued
-    int l_g = 0, l_blk = blockIdx.x + gi * gridDim.x, l_tab = 0;
+    int l_g = 0, l_blk = cid + gi * n_cl, l_tab = 0;
     const uint8_t* l_w[NPT];                                   // the lane's pieces at the cursor's group
 #pragma unroll
     for (int m = 0; m < NPT; m++) l_w[m] = nullptr;
@@ -229,9 +253,9 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
         // staged once per CTA, as in qmv_pipe.cuh; the group sums leave as three TF32 parts
         for (int i = threadIdx.x; i < 3 * xn * 8; i += NT) {                  // the zero tail of every column of every part
             const int col = i >> 3;
-            parts[col * gpad + groups + (i & 7)] = 0.0f;
+            parts[col * gpad + cg + (i & 7)] = 0.0f;
         }
-        const int cpr = K >> 3, total_chunks = T * cpr;
+        const int cpr = cg << (GSH - 3), total_chunks = T * cpr, k0 = gb << GSH;
         constexpr int cpg = GS / 8;
         constexpr int SU = 4;                                  // chunks whose loads are in flight together
         const bool f16_fast = (BITS == 4 || BITS == 8) && split == 1 && q.x_dtype == DT_F16;
@@ -242,7 +266,7 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
                 const int idx = base + u * NT + threadIdx.x;
                 if (idx < total_chunks) {
                     const int tok = tp.cpr_shift >= 0 ? idx >> tp.cpr_shift : idx / cpr, k = (idx - tok * cpr) * 8;
-                    load8_raw(q.x, q.x_dtype, static_cast<size_t>(tok) * q.x_stride + k, ra[u], rb[u]);
+                    load8_raw(q.x, q.x_dtype, static_cast<size_t>(tok) * q.x_stride + k0 + k, ra[u], rb[u]);
                 }
             }
 #pragma unroll
@@ -267,7 +291,7 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
                     if (q.x_up != nullptr) {
                         // gated input: the activation the layer sees is act(gate) * up, formed here
                         float up[8];
-                        load8_coherent(q.x_up, DT_F32, static_cast<size_t>(tok) * q.x_stride + k, up);
+                        load8_coherent(q.x_up, DT_F32, static_cast<size_t>(tok) * q.x_stride + k0 + k, up);
 #pragma unroll
                         for (int i = 0; i < 8; i++) v[i] = act_mul(q.x_act, v[i], up[i]);
                     }
@@ -313,9 +337,9 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
     for (int ps = 0; ps < NP; ps++) {
         const int col = ps * 8 + g;
         const bool valid = col < xn;
-        xb[ps] = valid ? smem_u32(xs) + (col * tp.xstride + gmin * GS + t * CL) * 2 : zaddr0;
+        xb[ps] = valid ? smem_u32(xs) + (col * tp.xstride + gl0 * GS + t * CL) * 2 : zaddr0;
         xinc[ps] = valid ? GS * 2 : 0;
-        sb_[ps] = valid ? smem_u32(parts) + (col * gpad + gmin + 2 * t) * 4 : zaddr0;
+        sb_[ps] = valid ? smem_u32(parts) + (col * gpad + gl0 + 2 * t) * 4 : zaddr0;
         sinc[ps] = valid ? 32u : 0u;                            // a window of eight group sums
         pstr[ps] = valid ? static_cast<uint32_t>(xn) * gpad * 4 : 0u;   // bytes between the parts of the group sums
         asm volatile("" : "+r"(xb[ps]), "+r"(sb_[ps]) :: "memory");
@@ -324,7 +348,22 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
     float* part_g = part + gi * tp.parities * par_floats;
     uint32_t c_src = ring;
     int c_tab = 0;
-    int c_blk = blockIdx.x + gi * gridDim.x;
+    int c_blk = cid + gi * n_cl;
+    // an output's row bias, gate and stores
+    auto finish = [&](int row, int tok, float v) {
+        if (row >= q.total_rows) return;
+        int pr = row, pi = 0;
+        if (q.n_parts > 1 && pr >= q.part[0].rows) {
+            pr -= q.part[0].rows; pi = 1;
+            if (q.n_parts > 2 && pr >= q.part[1].rows) { pr -= q.part[1].rows; pi = 2; }
+        }
+        if (q.has_bias) v += load_scalar(q.part[pi].bias, q.bias_dtype, pr);
+        if (q.e != nullptr) v = act_mul(q.act, v, __ldcg(q.e + row));
+        const size_t at = static_cast<size_t>(tok) * q.y_stride + row;
+        store_scalar(q.y, q.y_dtype, at, v);
+        for (int pp_ = 0; pp_ < q.peer.n; pp_++) store_scalar(q.peer.y[pp_], q.y_dtype, at, v);
+    };
+    float* zsum = reinterpret_cast<float*>(smem_tok + tp.off_z);
     for (int bj = 0; bj < my_blocks; bj++, c_blk += blk_stride) {
         float yacc[NP][4], yb[NP][4];
 #pragma unroll
@@ -472,33 +511,39 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
         // being read: it meets the others at the next block's barrier before it writes this parity again.  With a
         // single slot the group meets a second time, after the reads.)
         if (2 * kw < T) {
-            if (!peers_ready) {
+            if (kz == 1 && !peers_ready) {
                 if (lane < q.peer.n) peer_flag_wait(q.peer.my_flags + q.peer.peer_rank[lane], peer_epoch - 2u, p.err);
                 __syncwarp();
                 peers_ready = true;
             }
             for (int tok = 2 * kw + (lane >> 4); tok < T; tok += 2 * ks) {
                 const int r = lane & 15;
-                const int row = c_blk * 16 + r;
                 float v = 0.0f;
                 for (int wv = 0; wv < ks; wv++) v += slot_base[wv * (16 * TP) + r * TP + tok];
-                if (row < q.total_rows) {
-                    int pr = row, pi = 0;
-                    if (q.n_parts > 1 && pr >= q.part[0].rows) {
-                        pr -= q.part[0].rows; pi = 1;
-                        if (q.n_parts > 2 && pr >= q.part[1].rows) { pr -= q.part[1].rows; pi = 2; }
-                    }
-                    if (q.has_bias) v += load_scalar(q.part[pi].bias, q.bias_dtype, pr);
-                    if (q.e != nullptr) v = act_mul(q.act, v, __ldcg(q.e + row));
-                    const size_t at = static_cast<size_t>(tok) * q.y_stride + row;
-                    store_scalar(q.y, q.y_dtype, at, v);
-                    for (int pp_ = 0; pp_ < q.peer.n; pp_++) store_scalar(q.peer.y[pp_], q.y_dtype, at, v);
-                }
+                if (kz == 1) finish(c_blk * 16 + r, tok, v);
+                else zsum[((gi + bj * n_groups) * T + tok) * 16 + r] = v;
             }
         }
         if (tp.parities == 1 && ks > 1) asm volatile("bar.sync %0, %1;" ::"r"(1 + gi), "r"(ks * 32) : "memory");
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+
+    if (kz > 1) {
+        cluster_barrier();                                      // every CTA's sums are in its shared memory
+        if (!peers_ready) {
+            if (lane < q.peer.n) peer_flag_wait(q.peer.my_flags + q.peer.peer_rank[lane], peer_epoch - 2u, p.err);
+            __syncwarp();
+            peers_ready = true;
+        }
+        const uint32_t z = smem_u32(zsum);
+        for (int idx = rank * NT + threadIdx.x; idx < cta_blocks * T * 16; idx += kz * NT) {
+            float v = 0.0f;
+            for (int rk = 0; rk < kz; rk++) v += cluster_load(z + idx * 4, rk);
+            const int bt = idx >> 4, blk = bt / T;
+            finish((cid + blk * n_cl) * 16 + (idx & 15), bt - blk * T, v);
+        }
+        cluster_barrier();                                      // nobody leaves while its sums are being read
+    }
 
     if (q.peer.n > 0) peer_finish(q.peer, peer_epoch);
 }

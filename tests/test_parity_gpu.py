@@ -180,6 +180,22 @@ def test_small_batches_every_width_and_group(mlxq, oracle, bits):
 
 
 @pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
+def test_small_batches_of_long_rows(mlxq, oracle, bits):
+    # rows of 6144 codes and more are split over the CTAs of a cluster: even and uneven slices, fewer blocks than clusters
+    # and several rounds of them, 16 tokens of 16-bit activations (a wider cluster where the slices do not fit)
+    for gs, K, O, T, x_dtype in ((64, 6144, 41, 2, 0), (32, 6656, 600, 6, 0), (128, 12288, 24, 8, 0), (64, 14336, 40, 16, 1), (64, 6400, 700, 5, 2)):
+        fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=gs, scale_type=oracle.BF16, with_bias=(gs == 64), seed=bits + K)
+        layer = DevLayer.from_fixture(mlxq, fx)
+        x = oracle.RNG(T + K + bits).floats(T * K).reshape(T, K)
+        xr = as_dtype(x, x_dtype).float().cpu().numpy()
+        got = run(layer, x, T, x_dtype=x_dtype, x_stride=K + 8, y_stride=O + 5)
+        mlxq.streamStatus(None, 0)
+        # The bar of the small batches above holds for 1536 terms and is in units of max(1, |reference|): the rounding noise of
+        # a sum of K such terms is sqrt(K / 1536) times that.
+        close(oracle, got, fx.reference(xr), f"bits {bits} gs {gs} {O}x{K} T {T} x {x_dtype}", (1e-4 if x_dtype == 0 else 3e-5) * (K / 1536) ** 0.5)
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
 def test_one_fp32_token_every_width_and_group(mlxq, oracle, bits):
     # one fp32 token: its two fp16 parts on the kernel compiled for the group size, where slices of K hold whole drain
     # cycles of four groups, and on the general plan where they do not (K = 768); odd numbers of blocks and of steps
