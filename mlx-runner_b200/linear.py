@@ -113,15 +113,23 @@ class TensorView:
         return self.count * _DTYPE_SIZE[self.dtype]
 
 
+_TORCH_NAMES: dict = {}      # torch dtype -> element type name, filled when the first tensor is seen
+_TORCH_CODES: dict = {}      # torch dtype -> the C ABI's code, activation types only
+
+
 def _torch_dtype_name(t) -> str:
-    import torch
-    table = {torch.float32: "f32", torch.float16: "f16", torch.bfloat16: "bf16", torch.int32: "u32",
-             torch.uint8: "u8"}
-    if hasattr(torch, "uint32"):
-        table[torch.uint32] = "u32"
-    if t.dtype not in table:
+    if not _TORCH_NAMES:
+        import torch
+        table = {torch.float32: "f32", torch.float16: "f16", torch.bfloat16: "bf16", torch.int32: "u32",
+                 torch.uint8: "u8"}
+        if hasattr(torch, "uint32"):
+            table[torch.uint32] = "u32"
+        _TORCH_CODES.update({d: _DTYPE_CODE[n] for d, n in table.items() if n in _DTYPE_CODE})
+        _TORCH_NAMES.update(table)
+    name = _TORCH_NAMES.get(t.dtype)
+    if name is None:
         raise Unsupported(f"tensor dtype {t.dtype}")
-    return table[t.dtype]
+    return name
 
 
 def view(t) -> Optional[TensorView]:
@@ -133,26 +141,48 @@ def view(t) -> Optional[TensorView]:
     return TensorView(t.data_ptr(), _torch_dtype_name(t), tuple(t.shape), t)
 
 
+_raw_stream = None           # () -> the current stream's handle
+
+
+def _current_stream() -> int:
+    """``torch.cuda.current_stream().cuda_stream`` without the Stream object, which costs as much as a kernel launch; the
+    long form where this PyTorch has no such call."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        handle = torch.cuda.current_stream().cuda_stream         # (initialises CUDA)
+        raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+        if raw is not None and device is not None:
+            _raw_stream = lambda: raw(device())
+        else:
+            _raw_stream = lambda: torch.cuda.current_stream().cuda_stream
+        return handle
+    return _raw_stream()
+
+
 def _stream_handle(stream) -> int:
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        return _current_stream()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
 
 
 def _ptr(t) -> int:
+    data_ptr = getattr(t, "data_ptr", None)
+    if data_ptr is not None:
+        return data_ptr()
     if t is None:
         return 0
     if isinstance(t, int):
         return t
-    if isinstance(t, TensorView):
-        return t.ptr
-    return t.data_ptr()
+    return t.ptr
 
 
 def _act_dtype(t, default: Optional[int] = None) -> int:
+    code = _TORCH_CODES.get(getattr(t, "dtype", None))           # (a TensorView's dtype is a name: not found)
+    if code is not None:
+        return code
     if isinstance(t, TensorView):
         return _DTYPE_CODE[t.dtype]
     if isinstance(t, int):
