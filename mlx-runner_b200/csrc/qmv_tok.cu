@@ -25,7 +25,7 @@ bool supported(int bits, int gs) {
     return nm >= 2 && nm % 2 == 0;
 }
 
-template <int BITS, int GS, int NP, int DEPTH_CT>
+template <int BITS, int GS, int NP, int DEPTH_CT, bool CLUSTER>
 cudaError_t launch_one(const MmaParams& p, const TokPlan& tp, size_t smem, int device, cudaStream_t st) {
     if constexpr (!TokUnit<BITS, GS>::SUPPORTED) {
         return cudaErrorNotSupported;
@@ -37,7 +37,7 @@ cudaError_t launch_one(const MmaParams& p, const TokPlan& tp, size_t smem, int d
         {
             std::lock_guard<std::mutex> lk(mu);
             if (!done[device]) {
-                const cudaError_t e = cudaFuncSetAttribute(qmv_tok_kernel<BITS, GS, NP, DEPTH_CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_WHOLE);
+                const cudaError_t e = cudaFuncSetAttribute(qmv_tok_kernel<BITS, GS, NP, DEPTH_CT, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_WHOLE);
                 if (e != cudaSuccess) return e;
                 done[device] = true;
             }
@@ -51,7 +51,7 @@ cudaError_t launch_one(const MmaParams& p, const TokPlan& tp, size_t smem, int d
         la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         la[0].val.programmaticStreamSerializationAllowed = 1;
         int n = pdl_enabled() ? 1 : 0;
-        if (tp.kz > 1) {
+        if (CLUSTER) {
             la[n].id = cudaLaunchAttributeClusterDimension;
             la[n].val.clusterDim.x = static_cast<unsigned>(tp.kz);
             la[n].val.clusterDim.y = la[n].val.clusterDim.z = 1;
@@ -59,7 +59,7 @@ cudaError_t launch_one(const MmaParams& p, const TokPlan& tp, size_t smem, int d
         }
         cfg.attrs = la;
         cfg.numAttrs = static_cast<unsigned>(n);
-        return cudaLaunchKernelEx(&cfg, qmv_tok_kernel<BITS, GS, NP, DEPTH_CT>, p, tp);
+        return cudaLaunchKernelEx(&cfg, qmv_tok_kernel<BITS, GS, NP, DEPTH_CT, CLUSTER>, p, tp);
     }
 }
 
@@ -67,7 +67,8 @@ template <int BITS, int GS, int NP>
 cudaError_t launch_depth(const MmaParams& p, const TokPlan& tp, size_t smem, int device, cudaStream_t st) {
     // the width's usual ring depth is compiled in; a shallower ring (shared memory short) takes the general instance
     constexpr int usual = GS * BITS / 32 >= 16 ? 4 : 8;
-    return tp.depth == usual ? launch_one<BITS, GS, NP, usual>(p, tp, smem, device, st) : launch_one<BITS, GS, NP, 0>(p, tp, smem, device, st);
+    if (tp.kz > 1) return tp.depth == usual ? launch_one<BITS, GS, NP, usual, true>(p, tp, smem, device, st) : launch_one<BITS, GS, NP, 0, true>(p, tp, smem, device, st);
+    return tp.depth == usual ? launch_one<BITS, GS, NP, usual, false>(p, tp, smem, device, st) : launch_one<BITS, GS, NP, 0, false>(p, tp, smem, device, st);
 }
 
 template <int BITS, int GS>
@@ -95,7 +96,7 @@ int cluster_capacity(int kz, int sms) {
     const int slot = kz == 2 ? 0 : kz == 4 ? 1 : 2;
     std::lock_guard<std::mutex> lk(mu);
     if (!cached[dev][slot]) {
-        const auto kernel = qmv_tok_kernel<4, 64, 1, 4>;
+        const auto kernel = qmv_tok_kernel<4, 64, 1, 4, true>;
         int n = 0;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(sms / kz * kz));
