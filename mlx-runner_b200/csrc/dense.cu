@@ -35,45 +35,80 @@ __device__ __forceinline__ void load8_any(const void* p, int dt, size_t idx, boo
     for (int i = 0; i < 8; i++) o[i] = load_scalar(p, dt, idx + i);
 }
 
+// A warp takes ROWS rows: their weights are streamed once, and every activation it loads serves all of them.  (With
+// a row per warp the activations, read again for every row through L1, were the larger stream: 32000 x 4096 bf16 took
+// 86 / 105 / 164 / 310 us with 1 / 2 / 4 / 8 fp32 tokens.)  NT: tokens of the call, compiled in so that the accumulators
+// of absent tokens cost nothing.
+template <int NT, int ROWS>
 __global__ void __launch_bounds__(DENSE_WARPS * 32)
 dense_mv_kernel(const void* __restrict__ w, int w_dtype, const void* __restrict__ bias, int bias_dtype, const void* __restrict__ x,
-                int x_dtype, long long x_stride, void* __restrict__ y, int y_dtype, long long y_stride, int tt, int O, int K,
+                int x_dtype, long long x_stride, void* __restrict__ y, int y_dtype, long long y_stride, int O, int K,
                 int w_vec, int x_vec) {
     const int lane = threadIdx.x & 31;
-    const int row = blockIdx.x * DENSE_WARPS + (threadIdx.x >> 5);
-    if (row >= O) return;
-    float acc[DENSE_TOKENS];
+    const int row0 = (blockIdx.x * DENSE_WARPS + (threadIdx.x >> 5)) * ROWS;
+    if (row0 >= O) return;
+    float acc[ROWS][NT];
+    size_t wrow[ROWS];
 #pragma unroll
-    for (int t = 0; t < DENSE_TOKENS; t++) acc[t] = 0.0f;
-    const size_t wrow = static_cast<size_t>(row) * K;
+    for (int r = 0; r < ROWS; r++) {
+        wrow[r] = static_cast<size_t>(min(row0 + r, O - 1)) * K;      // (rows past the end read the last row; never stored)
+#pragma unroll
+        for (int t = 0; t < NT; t++) acc[r][t] = 0.0f;
+    }
     const int K8 = K & ~7;
+#pragma unroll(NT <= 2 && ROWS == 1 ? 4 : 2)
     for (int k = lane * 8; k < K8; k += 256) {
-        float wv[8];
-        load8_any(w, w_dtype, wrow + k, w_vec != 0, wv);
+        float wv[ROWS][8];
 #pragma unroll
-        for (int t = 0; t < DENSE_TOKENS; t++) {
-            if (t < tt) {
-                float xv[8];
-                load8_any(x, x_dtype, static_cast<size_t>(t) * x_stride + k, x_vec != 0, xv);
+        for (int r = 0; r < ROWS; r++) load8_any(w, w_dtype, wrow[r] + k, w_vec != 0, wv[r]);
 #pragma unroll
-                for (int i = 0; i < 8; i++) acc[t] = fmaf(wv[i], xv[i], acc[t]);
-            }
+        for (int t = 0; t < NT; t++) {
+            float xv[8];
+            load8_any(x, x_dtype, static_cast<size_t>(t) * x_stride + k, x_vec != 0, xv);
+#pragma unroll
+            for (int r = 0; r < ROWS; r++)
+#pragma unroll
+                for (int i = 0; i < 8; i++) acc[r][t] = fmaf(wv[r][i], xv[i], acc[r][t]);
         }
     }
     for (int k = K8 + lane; k < K; k += 32) {
-        const float wv = load_scalar(w, w_dtype, wrow + k);
-        for (int t = 0; t < tt; t++) acc[t] = fmaf(wv, load_scalar(x, x_dtype, static_cast<size_t>(t) * x_stride + k), acc[t]);
-    }
 #pragma unroll
-    for (int t = 0; t < DENSE_TOKENS; t++) {
-        float v = acc[t];
+        for (int r = 0; r < ROWS; r++) {
+            const float wv = load_scalar(w, w_dtype, wrow[r] + k);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0 && t < tt) {
-            if (bias != nullptr) v += load_scalar(bias, bias_dtype, row);
-            store_scalar(y, y_dtype, static_cast<size_t>(t) * y_stride + row, v);
+            for (int t = 0; t < NT; t++) acc[r][t] = fmaf(wv, load_scalar(x, x_dtype, static_cast<size_t>(t) * x_stride + k), acc[r][t]);
         }
     }
+#pragma unroll
+    for (int r = 0; r < ROWS; r++)
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+            float v = acc[r][t];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            const int row = row0 + r;
+            if (lane == 0 && row < O) {
+                if (bias != nullptr) v += load_scalar(bias, bias_dtype, row);
+                store_scalar(y, y_dtype, static_cast<size_t>(t) * y_stride + row, v);
+            }
+        }
+}
+
+template <int NT, int ROWS>
+void launch_tokens(int nt, unsigned grid, cudaStream_t st, const void* w, int w_dtype, const void* bias, int bias_dtype, const void* x, int x_dtype,
+                   long long x_stride, void* y, int y_dtype, long long y_stride, int O, int K, int w_vec, int x_vec) {
+    if constexpr (NT > 1)
+        if (nt < NT) return launch_tokens<NT - 1, ROWS>(nt, grid, st, w, w_dtype, bias, bias_dtype, x, x_dtype, x_stride, y, y_dtype, y_stride, O, K, w_vec, x_vec);
+    dense_mv_kernel<NT, ROWS><<<grid, DENSE_WARPS * 32, 0, st>>>(w, w_dtype, bias, bias_dtype, x, x_dtype, x_stride, y, y_dtype, y_stride, O, K, w_vec, x_vec);
+}
+
+// Rows per warp.  More of them save activation reads but leave fewer warps, which few rows or few tokens do not pay for
+// (1 / 2 / 4 rows per warp: 32000 x 4096 with 4 tokens 167 / 139 / 195 us, with 8 351 / 305 / 269; 4096 x 4096 with 2 tokens
+// 19 / 27 / 42, with 8 74 / 50 / 70; 2048 x 2048 with 8 tokens 21 / 24 / 32).
+int rows_per_warp(int tokens, int O) {
+    if (tokens >= 5) return O >= 24576 ? 4 : O >= 4096 ? 2 : 1;
+    if (tokens >= 2) return O >= (tokens == 2 ? 24576 : 8192) ? 2 : 1;
+    return 1;
 }
 
 }  // namespace
@@ -83,12 +118,13 @@ cudaError_t launch_dense(const void* w, int w_dtype, const void* bias, int bias_
     const size_t wsz = dtype_size(w_dtype), xsz = dtype_size(x_dtype);
     const int w_vec = (reinterpret_cast<uintptr_t>(w) % 16 == 0 && (static_cast<size_t>(K) * wsz) % 16 == 0) ? 1 : 0;
     const int x_vec = (reinterpret_cast<uintptr_t>(x) % 16 == 0 && (static_cast<size_t>(x_stride) * xsz) % 16 == 0) ? 1 : 0;
-    const unsigned grid = static_cast<unsigned>((O + DENSE_WARPS - 1) / DENSE_WARPS);
     for (long long t0 = 0; t0 < T; t0 += DENSE_TOKENS) {
         const int tt = static_cast<int>(T - t0 < DENSE_TOKENS ? T - t0 : DENSE_TOKENS);
-        dense_mv_kernel<<<grid, DENSE_WARPS * 32, 0, st>>>(
-            w, w_dtype, bias, bias_dtype, static_cast<const char*>(x) + static_cast<size_t>(t0) * x_stride * xsz, x_dtype, x_stride,
-            static_cast<char*>(y) + static_cast<size_t>(t0) * y_stride * dtype_size(y_dtype), y_dtype, y_stride, tt, O, K, w_vec, x_vec);
+        const int rows = rows_per_warp(tt, O);
+        const unsigned grid = static_cast<unsigned>((O + DENSE_WARPS * rows - 1) / (DENSE_WARPS * rows));
+        const auto launch = rows == 4 ? launch_tokens<DENSE_TOKENS, 4> : rows == 2 ? launch_tokens<DENSE_TOKENS, 2> : launch_tokens<DENSE_TOKENS, 1>;
+        launch(tt, grid, st, w, w_dtype, bias, bias_dtype, static_cast<const char*>(x) + static_cast<size_t>(t0) * x_stride * xsz, x_dtype, x_stride,
+               static_cast<char*>(y) + static_cast<size_t>(t0) * y_stride * dtype_size(y_dtype), y_dtype, y_stride, O, K, w_vec, x_vec);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
