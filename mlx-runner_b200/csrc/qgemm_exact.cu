@@ -112,31 +112,6 @@ template <int BYTES> __device__ __forceinline__ void cp_piece(uint32_t dst, cons
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// Whole-warp wait for two or three barriers (mbar_wait_warp of sm100_ptx.cuh with one poller and one broadcast for all: a
-// wait for a barrier that is complete already costs about 150 cycles, most of them around the poll).
-__device__ __forceinline__ bool wait_both(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1, int* abort_flag, unsigned* err) {
-    int got = 1;
-    if ((threadIdx.x & 31) == 0) got = mbar_wait(b0, p0, abort_flag, err) && mbar_wait(b1, p1, abort_flag, err) ? 1 : 0;
-    got = __shfl_sync(0xffffffffu, got, 0);
-    __syncwarp();
-    return got != 0;
-}
-__device__ __forceinline__ bool wait_three(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1, uint64_t* b2, uint32_t p2, int* abort_flag, unsigned* err) {
-    int got = 1;
-    if ((threadIdx.x & 31) == 0)
-        got = mbar_wait(b0, p0, abort_flag, err) && mbar_wait(b1, p1, abort_flag, err) && mbar_wait(b2, p2, abort_flag, err) ? 1 : 0;
-    got = __shfl_sync(0xffffffffu, got, 0);
-    __syncwarp();
-    return got != 0;
-}
-
-// one lane of a converged warp
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
-
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -270,7 +245,7 @@ qgemm_exact_kernel(const __grid_constant__ CUtensorMap map_x, const ExactArgs a)
                 const uint64_t x1 = x_desc + static_cast<uint64_t>(s * (XS * X_TILE / 16)), x2 = x1 + X_TILE / 16;
                 const uint32_t a_addr = tmem + A_COL0 + sa * 32;
                 for (int j = 0; j < spst; j++) {
-                    if (!wait_three(&bars->d_empty[buf], d_phase, &bars->full_x[s], (it / S_X) & 1, &bars->full_a[sa], (it / S_A) & 1,
+                    if (!mbar_wait_three(&bars->d_empty[buf], d_phase, &bars->full_x[s], (it / S_X) & 1, &bars->full_a[sa], (it / S_A) & 1,
                                     &bars->abort_flag, a.err)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t d_addr = tmem + buf * BN_MAX;
@@ -394,7 +369,7 @@ qgemm_exact_kernel(const __grid_constant__ CUtensorMap map_x, const ExactArgs a)
                 // the step's scales, biases and sums (copied by the producer, far ahead), then its products
                 const uint32_t sl = step % S_T;
                 const uint8_t* ts = t_ring + sl * T_SLOT;
-                if (!wait_both(&bars->full_t[sl], (step / S_T) & 1, &bars->d_full[buf], d_phase, &bars->abort_flag, a.err)) { ok = false; break; }
+                if (!mbar_wait_both(&bars->full_t[sl], (step / S_T) & 1, &bars->d_full[buf], d_phase, &bars->abort_flag, a.err)) { ok = false; break; }
                 tc_fence_after();
                 uint32_t d[NC];
 #pragma unroll

@@ -58,9 +58,10 @@ constexpr int X_STAGE = BN * BK * 2;    // 16384 bytes
 constexpr int W_SLAB = BM * 128;        // 32768 bytes: 256 rows x 128 bytes, 128-byte swizzle
 constexpr int NUM_THREADS = 20 * 32;
 constexpr int W_PRODUCER = 2;           // warp that streams the packed weight slabs
-// Two warps issue the MMAs, one per 128-row half of the tile (lane 0 of each).  A single thread needs ~110 cycles
-// per tcgen05.mma (operands travel through uniform registers) while an M128 N128 K16 MMA executes in 64: with one
-// issuer the tensor pipe was busy a third of the time.  The halves use separate accumulators and separate A
+// Two warps issue the MMAs, one per 128-row half of the tile.  From a branch that lane 0 takes alone an MMA cost ~110
+// cycles to issue (its operands travel through uniform registers) while an M128 N128 K16 MMA executes in 64.  The lanes
+// now stay together and elect one for the instruction, and one poll serves both barriers of a stage: 12288 x 4096 with
+// 1999 tokens 210.9 -> 198.2 us, 14336 x 4096 with 8192 tokens 880 -> 846 us.  The halves use separate accumulators and separate A
 // columns, so nothing orders the two issuers against each other; stage and accumulator barriers count both.
 constexpr int MMA_WARP = 1;             // issuer of half 0; it also owns the tensor-memory allocation
 constexpr int MMA_WARP2 = 3;            // issuer of half 1
@@ -125,7 +126,7 @@ qgemm4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     uint8_t* w_slabs = smem + S_X * X_STAGE;                   // S_W x 32 KB, each 1024-byte aligned
     Barriers* bars = reinterpret_cast<Barriers*>(smem + S_X * X_STAGE + S_W * W_SLAB);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int k_stages = a.K / BK;
     const int total_tiles = a.m_tiles * a.n_tiles;
 
@@ -147,7 +148,7 @@ qgemm4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base), 0);
     // Launched as a programmatic dependent of the pre-pass: the set-up above and the weight producer's first slabs
     // (the layer's constants) run while it finishes; every other role first waits for it (staged activations, the
     // scale/bias table, and -- through the pre-pass's own ordering -- everything earlier in the stream).
@@ -198,30 +199,29 @@ qgemm4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             }
         }
     } else if (warp == MMA_WARP || warp == MMA_WARP2) {
-        // ---- MMA issuers ------------------------------------------------------------------------------------
-        if (lane == 0) {
-            uint32_t it = 0, tile_i = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, tile_i++) {
-                if (tile_i > 0 && !mbar_wait(&bars->d_empty[warp == MMA_WARP ? 0 : 1], (tile_i - 1) & 1, &bars->abort_flag, a.err)) break;
+        // ---- MMA issuers: one per row half, the warp's lanes together, one elected for the instructions -------------------------
+        const int half = warp == MMA_WARP ? 0 : 1;
+        const uint32_t d_addr = tmem + D_COL0 + half * BN;
+        const uint64_t x_desc = smem_desc_sw128(smem_u32(x_tiles));
+        uint32_t it = 0, tile_i = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, tile_i++) {
+            if (tile_i > 0 && !mbar_wait_warp(&bars->d_empty[half], (tile_i - 1) & 1, &bars->abort_flag, a.err)) break;
+            for (int ks = 0; ks < k_stages; ks++, it++) {
+                const uint32_t s = it % S_X, sa = it % S_A;
+                if (!mbar_wait_both(&bars->full_x[s], (it / S_X) & 1, &bars->full_a[sa], (it / S_A) & 1, &bars->abort_flag, a.err)) { ok = false; break; }
                 tc_fence_after();
-                for (int ks = 0; ks < k_stages; ks++, it++) {
-                    const int s = it % S_X, sa = it % S_A;
-                    if (!mbar_wait(&bars->full_x[s], (it / S_X) & 1, &bars->abort_flag, a.err)) { ok = false; break; }
-                    if (!mbar_wait(&bars->full_a[sa], (it / S_A) & 1, &bars->abort_flag, a.err)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t bdesc = smem_desc_sw128(smem_u32(x_tiles + s * X_STAGE));
-                    {
-                        const int half = warp == MMA_WARP ? 0 : 1;
-                        const uint32_t d_addr = tmem + D_COL0 + half * BN;
+                const uint64_t bdesc = x_desc + static_cast<uint64_t>(s * (X_STAGE / 16));
+                const uint32_t a_addr = tmem + a_col(0, half, 0) + sa * BK;
+                if (elect_one()) {
 #pragma unroll
-                        for (int kk = 0; kk < BK / 16; kk++)
-                            tc_mma_ts(d_addr, tmem + a_col(sa, half, kk >> 1) + (kk & 1) * 8, bdesc + static_cast<uint64_t>(kk * 2), a.idesc, (ks | kk) != 0);
-                    }
+                    for (int kk = 0; kk < BK / 16; kk++)
+                        tc_mma_ts(d_addr, a_addr + kk * 8, bdesc + static_cast<uint64_t>(kk * 2), a.idesc, (ks | kk) != 0);
                     tc_commit(&bars->empty_x[s]);      // the activation tile of stage s is free again
                     tc_commit(&bars->empty_a[sa]);     // so is the A stage in tensor memory
+                    if (ks == k_stages - 1) tc_commit(&bars->d_full);      // accumulators of this tile are complete
                 }
-                if (ok) tc_commit(&bars->d_full);      // accumulators of this tile are complete
+                __syncwarp();
             }
         }
     } else if (warp >= DEQ_WARP0) {
@@ -405,21 +405,21 @@ qgemm4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 }
 
 
-// ---- the wide tile: 128 weight rows x 256 tokens -----------------------------------------------------------------
+// ---- the wide tile: 128 weight rows x 256 (or 128) tokens -----------------------------------------------------------------
 // Same pipeline, other tile.  Every dequantised weight now meets 256 tokens instead of 128, so the dequantisers
 // (the limiter of the 256 x 128 tile) do half the work per flop: a K stage is 128 rows x 64 codes, stored by
 // eight warps, and the sixteen dequantising warps take alternate stages.  Only one A block per stage lives in
 // tensor memory, so the A ring holds eight stages where the tall tile has four.  The accumulator is one
 // 128 x 256 fp32 block; two threads issue the MMAs, one per 128-token half (N = 128 each, separate columns,
 // separate halves of the activation tile).  Costs: 36 KB of operands per stage instead of 24 KB (L2 traffic),
-// and batches are padded to 256 tokens, so the tall tile stays in use for short batches.
+// and batches are padded to 256 tokens; batches of up to 128 take the same kernel with 128 tokens a tile, or the tall tile
+// (see use_tall).
 namespace wide {
 
-constexpr int BM = 128, BN = 256;
-constexpr int S_X = 4;                  // activation stages of 32 KB
+constexpr int BM = 128;
+constexpr int S_X = 4;                  // activation stages of BN x 128 bytes
 constexpr int S_W = 3;                  // weight slabs of 16 KB (128 rows x 128 bytes = W_SPAN stages)
 constexpr int S_A = 8;                  // TMEM stages of the A operand, 32 columns each
-constexpr int X_STAGE = BN * BK * 2;    // 32768
 constexpr int W_SLAB = BM * 128;        // 16384
 constexpr int D_COL0 = 0, A_COL0 = 256;
 constexpr int STAGE_WARPS = DEQ_WARPS / 2;   // warps that store one stage
@@ -439,17 +439,19 @@ struct Barriers {
     int abort_flag;
 };
 
-constexpr int SMEM_BYTES = S_X * X_STAGE + S_W * W_SLAB + sizeof(Barriers) + 1024;
+template <int BN> constexpr int SMEM_BYTES = S_X * BN * BK * 2 + S_W * W_SLAB + static_cast<int>(sizeof(Barriers)) + 1024;
 
+template <int BN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 qgemm4w_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GemmArgs a) {
+    constexpr int X_STAGE = BN * BK * 2, HALF = BN / 2;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint8_t* x_tiles = smem;
     uint8_t* w_slabs = smem + S_X * X_STAGE;
     Barriers* bars = reinterpret_cast<Barriers*>(smem + S_X * X_STAGE + S_W * W_SLAB);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int k_stages = a.K / BK;
     const int total_tiles = a.m_tiles * a.n_tiles;
 
@@ -471,7 +473,7 @@ qgemm4w_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base), 0);
     // Launched as a programmatic dependent of the pre-pass: the set-up above and the weight producer's first slabs
     // (the layer's constants) run while it finishes; every other role first waits for it (staged activations, the
     // scale/bias table, and -- through the pre-pass's own ordering -- everything earlier in the stream).
@@ -520,29 +522,30 @@ qgemm4w_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             }
         }
     } else if (warp == MMA_WARP || warp == MMA_WARP2) {
-        // ---- MMA issuers: one per 128-token half of the tile ------------------------------------------------------------
-        if (lane == 0) {
-            const int nh = warp == MMA_WARP ? 0 : 1;
-            const uint32_t d_addr = tmem + D_COL0 + nh * 128;
-            uint32_t it = 0, tile_i = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, tile_i++) {
-                if (tile_i > 0 && !mbar_wait(&bars->d_empty[nh], (tile_i - 1) & 1, &bars->abort_flag, a.err)) break;
+        // ---- MMA issuers: one per half of the tile's tokens, the warp's lanes together, one elected for the instructions ------
+        const int nh = warp == MMA_WARP ? 0 : 1;
+        const uint32_t d_addr = tmem + D_COL0 + nh * HALF;
+        // this half's tokens are the second half of the stage (rows of 128 bytes, same swizzle phase)
+        const uint64_t x_desc = smem_desc_sw128(smem_u32(x_tiles + nh * (HALF * 128)));
+        uint32_t it = 0, tile_i = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, tile_i++) {
+            if (tile_i > 0 && !mbar_wait_warp(&bars->d_empty[nh], (tile_i - 1) & 1, &bars->abort_flag, a.err)) break;
+            for (int ks = 0; ks < k_stages; ks++, it++) {
+                const uint32_t s = it % S_X, sa = it % S_A;
+                if (!mbar_wait_both(&bars->full_x[s], (it / S_X) & 1, &bars->full_a[sa], (it / S_A) & 1, &bars->abort_flag, a.err)) { ok = false; break; }
                 tc_fence_after();
-                for (int ks = 0; ks < k_stages; ks++, it++) {
-                    const int s = it % S_X, sa = it % S_A;
-                    if (!mbar_wait(&bars->full_x[s], (it / S_X) & 1, &bars->abort_flag, a.err)) { ok = false; break; }
-                    if (!mbar_wait(&bars->full_a[sa], (it / S_A) & 1, &bars->abort_flag, a.err)) { ok = false; break; }
-                    tc_fence_after();
-                    // this half's 128 tokens are the second 16 KB of the stage (rows of 128 bytes, same swizzle phase)
-                    const uint64_t bdesc = smem_desc_sw128(smem_u32(x_tiles + s * X_STAGE + nh * (128 * 128)));
+                const uint64_t bdesc = x_desc + static_cast<uint64_t>(s * (X_STAGE / 16));
+                const uint32_t a_addr = tmem + a_col(0, 0) + sa * 32;
+                if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < BK / 16; kk++)
-                        tc_mma_ts(d_addr, tmem + a_col(sa, kk >> 1) + (kk & 1) * 8, bdesc + static_cast<uint64_t>(kk * 2), a.idesc, (ks | kk) != 0);
+                        tc_mma_ts(d_addr, a_addr + kk * 8, bdesc + static_cast<uint64_t>(kk * 2), a.idesc, (ks | kk) != 0);
                     tc_commit(&bars->empty_x[s]);
                     tc_commit(&bars->empty_a[sa]);
+                    if (ks == k_stages - 1) tc_commit(&bars->d_full);
                 }
-                if (ok) tc_commit(&bars->d_full);
+                __syncwarp();
             }
         }
     } else if (warp >= DEQ_WARP0) {
@@ -557,8 +560,8 @@ qgemm4w_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const __half2 kSub = __halves2half2(__float2half(-64.0f), __float2half(-64.0f));
         uint32_t it = 0, wi = 0, tile_i = 0;
         bool ok = true;
-        // Epilogue: this warp drains its lane quadrant for 64 of the 256 token columns.
-        const int e_cols = (dw >> 2) * 64, e_nh = dw >> 3;
+        // Epilogue: this warp drains its lane quadrant for a quarter of the token columns.
+        const int e_cols = (dw >> 2) * (BN / 4), e_nh = dw >> 3;
         auto epilogue = [&](int tile, uint32_t index) {
             const int row = (tile % a.m_tiles) * BM + r;
             const int tok0 = (tile / a.m_tiles) * BN + e_cols;
@@ -566,12 +569,12 @@ qgemm4w_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             tc_fence_after();
             const float rb = (a.bias != nullptr && row < a.O) ? load_scalar(a.bias, a.bias_dtype, row) : 0.0f;
 #pragma unroll 1
-            for (int c = 0; c < 2; c++) {
+            for (int c = 0; c < BN / 128; c++) {
                 uint32_t v[32];
                 __syncwarp();
                 tc_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + D_COL0 + e_cols + c * 32, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (c == 1) {
+                if (c == BN / 128 - 1) {
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&bars->d_empty[e_nh]);
@@ -858,8 +861,16 @@ bool gemm_map_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t oute
     return make_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_UINT16, base, inner, outer, row_bytes, box_inner, box_outer, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-// Batches of more than 128 tokens take the wide tile (128 rows x 256 tokens), shorter ones the tall one (256 x 128).
+// Batches of more than 128 tokens take the wide tile (128 rows x 256 tokens).  Shorter ones, where a tile's time is its K
+// loop whatever its rows, take 128 rows x 128 tokens (about 3/4 of the time of 256 x 128: 4096 x 4096 with 77 tokens 35
+// us against 47) unless the tall tile needs so many fewer rounds of the SMs that it is done first (28672 x 4096: 50 us
+// against 70).  The sums of an output are the same in every tile.
 static bool use_wide(long long T) { return T > 128; }
+static bool use_tall(long long T, int O, int sms) {
+    if (use_wide(T)) return false;
+    const int low = ((O + 127) / 128 + sms - 1) / sms, high = ((O + 255) / 256 + sms - 1) / sms;
+    return 4 * high < 3 * low;
+}
 
 int qgemm_tile_tokens(const GemmLayer& L, int x_dtype, long long x_stride, const void* x, long long T) {
     if (L.bits != 4 || L.K % BK != 0 || L.K < 2 * S_A * BK || L.gs < 32 || (L.gs & (L.gs - 1)) != 0 || L.O < 1 || T < 1) return 0;
@@ -867,7 +878,7 @@ int qgemm_tile_tokens(const GemmLayer& L, int x_dtype, long long x_stride, const
     if ((reinterpret_cast<uintptr_t>(L.w) & 15u) != 0) return 0;
     if (x != nullptr && ((reinterpret_cast<uintptr_t>(x) & 15u) != 0 || (x_stride * 2) % 16 != 0)) return 0;
     if (T > 0x7FFFFFFFLL) return 0;
-    return use_wide(T) ? wide::BN : BN;
+    return use_wide(T) ? 256 : 128;
 }
 
 namespace {
@@ -892,7 +903,9 @@ cudaError_t gemm_attr(int device) {
     if (!done[device]) {
         cudaError_t e = cudaFuncSetAttribute(qgemm4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
         if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(wide::qgemm4w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide::SMEM_BYTES);
+        e = cudaFuncSetAttribute(wide::qgemm4w_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, wide::SMEM_BYTES<256>);
+        if (e != cudaSuccess) return e;
+        e = cudaFuncSetAttribute(wide::qgemm4w_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, wide::SMEM_BYTES<128>);
         if (e != cudaSuccess) return e;
         done[device] = true;
     }
@@ -908,8 +921,8 @@ cudaError_t enqueue_gemm(const GemmLayer& L, const GemmCall& c, cudaStream_t st,
     a.O = L.O; a.K = L.K; a.gs = L.gs; a.T = static_cast<int>(c.T);
     a.gs_shift = 0;
     while ((1 << a.gs_shift) < L.gs) a.gs_shift++;
-    const bool wide_tile = use_wide(c.T);
-    const int bm = wide_tile ? wide::BM : BM, bn = wide_tile ? wide::BN : BN;
+    const bool wide_tile = use_wide(c.T), tall = use_tall(c.T, L.O, sm_count(L.device));
+    const int bm = tall ? BM : wide::BM, bn = wide_tile ? 256 : 128;
     a.m_tiles = (L.O + bm - 1) / bm;
     a.n_tiles = static_cast<int>((c.T + bn - 1) / bn);
     const bool have_table = c.table != nullptr;
@@ -941,20 +954,21 @@ cudaError_t enqueue_gemm(const GemmLayer& L, const GemmCall& c, cudaStream_t st,
     }
     // instruction descriptor: fp32 accumulate (bit 4), A and B fp16 (format 0 at bits 7 and 10), both K-major,
     // N >> 3 at bit 17, M >> 4 at bit 24
-    a.idesc = (1u << 4) | (0u << 7) | (0u << 10) | (static_cast<uint32_t>(128 >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
+    a.idesc = (1u << 4) | (0u << 7) | (0u << 10) | (static_cast<uint32_t>((tall ? 128 : bn / 2) >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
     const long long tiles = static_cast<long long>(a.m_tiles) * a.n_tiles;
     const int sms = sm_count(L.device);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(tiles < sms ? tiles : sms));
     cfg.blockDim = dim3(NUM_THREADS);
-    cfg.dynamicSmemBytes = wide_tile ? wide::SMEM_BYTES : SMEM_BYTES;
+    cfg.dynamicSmemBytes = tall ? SMEM_BYTES : wide_tile ? wide::SMEM_BYTES<256> : wide::SMEM_BYTES<128>;
     cfg.stream = st;
     cudaLaunchAttribute la[1];
     la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;       // a dependent of the pre-pass, see the kernels
     la[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = la;
     cfg.numAttrs = 1;
-    if (wide_tile) return cudaLaunchKernelEx(&cfg, wide::qgemm4w_kernel, map_w, map_x, a);
+    if (wide_tile) return cudaLaunchKernelEx(&cfg, wide::qgemm4w_kernel<256>, map_w, map_x, a);
+    if (!tall) return cudaLaunchKernelEx(&cfg, wide::qgemm4w_kernel<128>, map_w, map_x, a);
     return cudaLaunchKernelEx(&cfg, qgemm4_kernel, map_w, map_x, a);
 }
 

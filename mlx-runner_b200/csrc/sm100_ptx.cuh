@@ -85,6 +85,31 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, i
     return got != 0;
 }
 
+// Whole-warp wait for two or three barriers (mbar_wait_warp above with one poller and one broadcast for all: a
+// wait for a barrier that is complete already costs about 150 cycles, most of them around the poll).
+__device__ __forceinline__ bool mbar_wait_both(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1, int* abort_flag, unsigned* err) {
+    int got = 1;
+    if ((threadIdx.x & 31) == 0) got = mbar_wait(b0, p0, abort_flag, err) && mbar_wait(b1, p1, abort_flag, err) ? 1 : 0;
+    got = __shfl_sync(0xffffffffu, got, 0);
+    __syncwarp();
+    return got != 0;
+}
+__device__ __forceinline__ bool mbar_wait_three(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1, uint64_t* b2, uint32_t p2, int* abort_flag, unsigned* err) {
+    int got = 1;
+    if ((threadIdx.x & 31) == 0)
+        got = mbar_wait(b0, p0, abort_flag, err) && mbar_wait(b1, p1, abort_flag, err) && mbar_wait(b2, p2, abort_flag, err) ? 1 : 0;
+    got = __shfl_sync(0xffffffffu, got, 0);
+    __syncwarp();
+    return got != 0;
+}
+
+// one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
