@@ -36,6 +36,7 @@
 
 #include "mlxq_device.cuh"
 #include "qgemm_exact.cuh"
+#include "qmv_pipe.cuh"
 #include "sm100_ptx.cuh"
 
 namespace mlxq {
@@ -465,6 +466,7 @@ struct ExactStage {
 
 __global__ void __launch_bounds__(256) exact_stage_kernel(const ExactStage g) {
     if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");           // a dependent of the previous kernel; what that wrote is read through L2
     if (blockIdx.x < g.x_blocks) {
         const int chunks = g.K / 8;                              // a multiple of 16
         const long long n = static_cast<long long>(g.T) * chunks;
@@ -475,9 +477,7 @@ __global__ void __launch_bounds__(256) exact_stage_kernel(const ExactStage g) {
             const int t = live ? static_cast<int>(i / chunks) : 0, c = live ? static_cast<int>(i - static_cast<long long>(t) * chunks) : 0;
             const size_t at = static_cast<size_t>(t) * g.x_stride + c * 8;
             float v[8];
-            if (g.x_dtype == DT_F32) XLoad<float>::load8(static_cast<const float*>(g.x) + at, v);
-            else if (g.x_dtype == DT_F16) XLoad<__half>::load8(static_cast<const __half*>(g.x) + at, v);
-            else XLoad<__nv_bfloat16>::load8(static_cast<const __nv_bfloat16*>(g.x) + at, v);
+            load8_coherent(g.x, g.x_dtype, at, v);
             float sum = 0.0f;
 #pragma unroll
             for (int j = 0; j < 8; j++) sum += v[j];
@@ -668,8 +668,16 @@ cudaError_t launch_qgemm_exact(const GemmLayer& L, const GemmCall& c, cudaStream
         const long long nx = (static_cast<long long>(T) * (L.K / 8) + 255) / 256;
         const long long ns = (static_cast<long long>((groups + 7) / 8) * o_pad + 255) / 256;
         g.x_blocks = static_cast<unsigned>(nx < 148 * 6 ? nx : 148 * 6);
-        exact_stage_kernel<<<g.x_blocks + static_cast<unsigned>(ns < 148 * 4 ? ns : 148 * 4), 256, 0, st>>>(g);
-        err = cudaGetLastError();
+        cudaLaunchConfig_t sc = {};
+        sc.gridDim = dim3(g.x_blocks + static_cast<unsigned>(ns < 148 * 4 ? ns : 148 * 4));
+        sc.blockDim = dim3(256);
+        sc.stream = st;
+        cudaLaunchAttribute sa[1];
+        sa[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        sa[0].val.programmaticStreamSerializationAllowed = 1;
+        sc.attrs = sa;
+        sc.numAttrs = 1;
+        err = cudaLaunchKernelEx(&sc, exact_stage_kernel, g);
         if (err != cudaSuccess) { *why = "pre-pass"; break; }
         CUtensorMap map_x;
         if (!gemm_map_2d(&map_x, xs, static_cast<uint64_t>(L.K), static_cast<uint64_t>(T) * parts, static_cast<uint64_t>(L.K) * 2, BK, bn)) {

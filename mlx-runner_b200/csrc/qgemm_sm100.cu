@@ -131,6 +131,7 @@ qgemm4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     const int total_tiles = a.m_tiles * a.n_tiles;
 
     if (threadIdx.x == 0) {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // (the next call's pre-pass may be resident early)
         for (int i = 0; i < S_X; i++) { mbar_init(&bars->full_x[i], 1); mbar_init(&bars->empty_x[i], 2); }
         for (int i = 0; i < S_W; i++) { mbar_init(&bars->full_w[i], 1); mbar_init(&bars->empty_w[i], DEQ_WARPS); }
         for (int i = 0; i < S_A; i++) { mbar_init(&bars->full_a[i], DEQ_WARPS); mbar_init(&bars->empty_a[i], 2); }
@@ -417,7 +418,9 @@ qgemm4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 namespace wide {
 
 constexpr int BM = 128;
-constexpr int S_X = 4;                  // activation stages of BN x 128 bytes
+// activation stages of BN x 128 bytes: 128 KB in flight either way (64 KB left the MMAs of the small tile waiting)
+template <int BN> constexpr int X_STAGES = BN == 256 ? 4 : 8;
+constexpr int MAX_X_STAGES = 8;
 constexpr int S_W = 3;                  // weight slabs of 16 KB (128 rows x 128 bytes = W_SPAN stages)
 constexpr int S_A = 8;                  // TMEM stages of the A operand, 32 columns each
 constexpr int W_SLAB = BM * 128;        // 16384
@@ -427,8 +430,8 @@ constexpr int STAGE_WARPS = DEQ_WARPS / 2;   // warps that store one stage
 __host__ __device__ constexpr uint32_t a_col(int sa, int khalf) { return A_COL0 + static_cast<uint32_t>(sa * 32 + khalf * 16); }
 
 struct Barriers {
-    uint64_t full_x[S_X];
-    uint64_t empty_x[S_X];
+    uint64_t full_x[MAX_X_STAGES];
+    uint64_t empty_x[MAX_X_STAGES];
     uint64_t full_w[S_W];
     uint64_t empty_w[S_W];
     uint64_t full_a[S_A];
@@ -439,12 +442,12 @@ struct Barriers {
     int abort_flag;
 };
 
-template <int BN> constexpr int SMEM_BYTES = S_X * BN * BK * 2 + S_W * W_SLAB + static_cast<int>(sizeof(Barriers)) + 1024;
+template <int BN> constexpr int SMEM_BYTES = X_STAGES<BN> * BN * BK * 2 + S_W * W_SLAB + static_cast<int>(sizeof(Barriers)) + 1024;
 
 template <int BN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 qgemm4w_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GemmArgs a) {
-    constexpr int X_STAGE = BN * BK * 2, HALF = BN / 2;
+    constexpr int X_STAGE = BN * BK * 2, HALF = BN / 2, S_X = X_STAGES<BN>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint8_t* x_tiles = smem;
@@ -456,6 +459,7 @@ qgemm4w_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const int total_tiles = a.m_tiles * a.n_tiles;
 
     if (threadIdx.x == 0) {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // (the next call's pre-pass may be resident early)
         for (int i = 0; i < S_X; i++) { mbar_init(&bars->full_x[i], 1); mbar_init(&bars->empty_x[i], 2); }
         for (int i = 0; i < S_W; i++) { mbar_init(&bars->full_w[i], 1); mbar_init(&bars->empty_w[i], DEQ_WARPS); }
         for (int i = 0; i < S_A; i++) { mbar_init(&bars->full_a[i], STAGE_WARPS); mbar_init(&bars->empty_a[i], 2); }
@@ -714,7 +718,7 @@ __device__ __forceinline__ void stage_x_part(const uint16_t* __restrict__ x, int
     for (long long i = block * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<long long>(blocks) * blockDim.x) {
         const long long t = i / chunks, c = i - t * chunks;
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(x + t * x_stride + c * 8));
+        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(x + t * x_stride + c * 8));     // (written while this grid was resident)
         uint32_t w[4] = {v.x, v.y, v.z, v.w};
         if (is_bf16) {
 #pragma unroll
@@ -784,6 +788,8 @@ __global__ void stage_inputs_kernel(const StageArgs g) {
     // the GEMM that follows is launched as a programmatic dependent: it may set up (barriers, tensor memory, first
     // weight slabs) while this grid runs, and waits for this grid before it touches what is written here
     if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // ... and is itself a dependent of the stream's previous kernel: it neither reads nor writes anything before that is done
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (blockIdx.x < g.x_blocks) stage_x_part(g.x, g.is_bf16, g.x_stride, g.xs, g.T, g.K, blockIdx.x, g.x_blocks);
     else stage_scales_part(g.s, g.b, g.s_dtype, g.O, g.o_pad, g.gpr, g.gs_shift, g.k_stages, g.n_slabs, g.pairs,
                            blockIdx.x - g.x_blocks, gridDim.x - g.x_blocks);
@@ -939,7 +945,17 @@ cudaError_t enqueue_gemm(const GemmLayer& L, const GemmCall& c, cudaStream_t st,
         g.x_blocks = static_cast<unsigned>(n / 256 + 1 < 148LL * 6 ? n / 256 + 1 : 148LL * 6);
         // (the table part is left out when the layer's table was built ahead)
         const unsigned s_blocks = have_table ? 0u : static_cast<unsigned>(ns / 256 + 1 < 148LL * 4 ? ns / 256 + 1 : 148LL * 4);
-        stage_inputs_kernel<<<g.x_blocks + s_blocks, 256, 0, st>>>(g);
+        cudaLaunchConfig_t sc = {};
+        sc.gridDim = dim3(g.x_blocks + s_blocks);
+        sc.blockDim = dim3(256);
+        sc.stream = st;
+        cudaLaunchAttribute sa[1];
+        sa[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        sa[0].val.programmaticStreamSerializationAllowed = 1;
+        sc.attrs = sa;
+        sc.numAttrs = 1;
+        const cudaError_t se = cudaLaunchKernelEx(&sc, stage_inputs_kernel, g);
+        if (se != cudaSuccess) { *why = "pre-pass"; return se; }
     }
     CUtensorMap map_w, map_x;
     if (!make_map_2d(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, L.w, static_cast<uint64_t>(L.K) / 2, static_cast<uint64_t>(L.O),
