@@ -137,8 +137,10 @@ MLXQ_API int mlxq_linear_forward(mlxq_linear_t h, mlxq_stream_t stream, const vo
  * cudaFree or other allocating routine is called, and results are the same as mlxq_linear_forward's.
  *   - Batches with T * in_dim * 2 above 32 MiB, and layers with out_dim * in_dim / 8 above 16 MiB (rows
  *     rounded up to 256), are rejected with MLXQ_INVALID_ARGUMENT (split the batch; shard the layer).
- *   - Batches the GEMM does not take (T <= 16, fp32 activations, other bit widths) run on kernels that use no
- *     scratch memory, exactly as in mlxq_linear_forward.
+ *   - Batches the 4-bit GEMM does not take (T <= 16, fp32 activations, other bit widths) run on kernels that use no
+ *     scratch memory.  Beyond 16 tokens mlxq_linear_forward has a GEMM for them that does (and is much faster): there
+ *     the two agree to the fp32 rounding of their sums, not bit for bit.  The same holds between a batch encoded while
+ *     its stream is captured, which keeps these kernels, and one that is not.
  *   - Every call on a device shares the one array, which keeps whatever the last call wrote: calls that
  *     overlap on the GPU (different streams) race; order them on one stream or with events.
  *   - The first call on each device looks up the array's device address and sets the kernel's shared-memory

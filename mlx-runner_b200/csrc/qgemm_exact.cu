@@ -26,6 +26,10 @@
 // Split K.  A layer of few rows leaves most SMs without a tile, so K is cut into `S` segments worked on by different
 // CTAs; the warp that finishes a piece of the tile last adds the segments' partial sums in their order.  S depends on
 // the layer alone, not on the batch: a token's result is the same whatever batch it rides in.
+// Measured (pre-pass included, one decode-kernel pass per eight tokens before): 12288 x 4096, 4 bits, 512 fp32 tokens
+// 1398 -> 165 us (312 TFLOP/s counted once per term); 8 bits, 384 bf16 tokens 717 -> 121 us.  What bounds it now is the
+// drain: 128 x 128 sums leave tensor memory per 64 codes, two packed FMAs per pair of them, some 1700 cycles a stage
+// against 512 of the MMAs.
 // Every wait is bounded: a wait that runs out sets the device error word, raises the CTA's abort flag and all roles
 // fall through to the common exit, where tensor memory is released.
 #include <cuda.h>

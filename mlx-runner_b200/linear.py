@@ -280,7 +280,8 @@ class Linear:
     def encodeStatic(self, stream, x, xStride: int, y, yStride: int, T: int, xDtype: Optional[int] = None,
                      yDtype: Optional[int] = None) -> None:
         """``encode`` for hosts that must not allocate device memory while they run: the GEMM's staged copy
-        of the activations goes into the library's fixed 32 MiB array instead of pool memory.  Same results;
+        of the activations goes into the library's fixed 32 MiB array instead of pool memory.  Same results
+        (long batches that the 4-bit GEMM does not take: to fp32 rounding, on slower kernels without scratch);
         batches with ``T * inDim * 2`` bytes above the array are refused (``InvalidArgument``); calls that
         overlap on the GPU share the array and race.  No counterpart in the reference."""
         check(L.load().mlxq_linear_forward_static(self._h, _stream_handle(stream), _ptr(x), _act_dtype(x, xDtype),
