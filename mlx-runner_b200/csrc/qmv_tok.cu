@@ -51,7 +51,7 @@ cudaError_t launch_one(const MmaParams& p, const TokPlan& tp, size_t smem, int d
         la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         la[0].val.programmaticStreamSerializationAllowed = 1;
         int n = pdl_enabled() ? 1 : 0;
-        if (CLUSTER) {
+        if (tp.kz > 1) {
             la[n].id = cudaLaunchAttributeClusterDimension;
             la[n].val.clusterDim.x = static_cast<unsigned>(tp.kz);
             la[n].val.clusterDim.y = la[n].val.clusterDim.z = 1;
@@ -67,8 +67,10 @@ template <int BITS, int GS, int NP>
 cudaError_t launch_depth(const MmaParams& p, const TokPlan& tp, size_t smem, int device, cudaStream_t st) {
     // the width's usual ring depth is compiled in; a shallower ring (shared memory short) takes the general instance
     constexpr int usual = GS * BITS / 32 >= 16 ? 4 : 8;
-    if (tp.kz > 1) return tp.depth == usual ? launch_one<BITS, GS, NP, usual, true>(p, tp, smem, device, st) : launch_one<BITS, GS, NP, 0, true>(p, tp, smem, device, st);
-    return tp.depth == usual ? launch_one<BITS, GS, NP, usual, false>(p, tp, smem, device, st) : launch_one<BITS, GS, NP, 0, false>(p, tp, smem, device, st);
+    if (tp.kz > 1 || !planned_width<BITS>()) return tp.depth == usual ? launch_one<BITS, GS, NP, usual, true>(p, tp, smem, device, st) : launch_one<BITS, GS, NP, 0, true>(p, tp, smem, device, st);
+    if constexpr (planned_width<BITS>())
+        return tp.depth == usual ? launch_one<BITS, GS, NP, usual, false>(p, tp, smem, device, st) : launch_one<BITS, GS, NP, 0, false>(p, tp, smem, device, st);
+    return cudaErrorNotSupported;
 }
 
 template <int BITS, int GS>

@@ -97,7 +97,9 @@ __device__ __forceinline__ float cluster_load(uint32_t addr, int rank) {
 }
 
 // DEPTH_CT: the ring depth when it is the width's usual one (compiled in), 0 when the planner had to take a shallower ring.
-// CLUSTER: K is split over the CTAs of a cluster (compiled out otherwise: the extra code cost single CTAs 0.7 %).
+// CLUSTER: K may be split over the CTAs of a cluster.  Compiled out for single CTAs at the widths whose codes straddle bytes,
+// where the extra code cost 0.8 %; at the others the one instance serves both and is the faster one (step of 36 4-bit
+// layers, 6 tokens: 3343 us against 3407 with an instance for each).
 template <int BITS, int GS, int NP, int DEPTH_CT, bool CLUSTER>
 __global__ void __launch_bounds__(TOK_WARPS * 32, 1)
 qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokPlan tp) {
@@ -129,7 +131,7 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
     const int ks = tp.ks, gi = warp >> tp.ks_shift, kw = warp & (ks - 1), n_groups = TOK_WARPS >> tp.ks_shift;
     // the CTA's slice of K: groups [gb, gb + cg); the warp's: [gmin, gmin + slice_groups) of those.  Both are cut at even
     // groups so that (scale, bias) pairs stay whole.
-    const int kz_shift = CLUSTER ? tp.kz_shift : 0, kz = 1 << kz_shift;
+    const int kz_shift = CLUSTER ? tp.kz_shift : 0, kz = CLUSTER ? tp.kz : 1;
     const int rank = blockIdx.x & (kz - 1), cid = blockIdx.x >> kz_shift, n_cl = gridDim.x >> kz_shift;
     const int gb = CLUSTER ? (((groups >> 1) * rank) >> kz_shift) << 1 : 0;
     const int cg = CLUSTER ? ((((groups >> 1) * (rank + 1)) >> kz_shift) << 1) - gb : groups;
@@ -513,7 +515,7 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
         // being read: it meets the others at the next block's barrier before it writes this parity again.  With a
         // single slot the group meets a second time, after the reads.)
         if (2 * kw < T) {
-            if (!CLUSTER && !peers_ready) {
+            if ((!CLUSTER || kz == 1) && !peers_ready) {
                 if (lane < q.peer.n) peer_flag_wait(q.peer.my_flags + q.peer.peer_rank[lane], peer_epoch - 2u, p.err);
                 __syncwarp();
                 peers_ready = true;
@@ -522,7 +524,7 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
                 const int r = lane & 15;
                 float v = 0.0f;
                 for (int wv = 0; wv < ks; wv++) v += slot_base[wv * (16 * TP) + r * TP + tok];
-                if constexpr (!CLUSTER) finish(c_blk * 16 + r, tok, v);
+                if (!CLUSTER || kz == 1) finish(c_blk * 16 + r, tok, v);
                 else zsum[((gi + bj * n_groups) * T + tok) * 16 + r] = v;
             }
         }
@@ -530,7 +532,7 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 
-    if constexpr (CLUSTER) {
+    if (CLUSTER && kz > 1) {
         cluster_barrier();                                      // every CTA's sums are in its shared memory
         if (!peers_ready) {
             if (lane < q.peer.n) peer_flag_wait(q.peer.my_flags + q.peer.peer_rank[lane], peer_epoch - 2u, p.err);
