@@ -6,8 +6,9 @@
 // the rows were too long for it -- the whole layer was read and unpacked again for every eight tokens.
 //
 // Operands.  The A operand is the raw codes, centred: q - 2^(bits-1) is exact in fp16, and unpacking costs three to five
-// instructions per pair of codes.  16-bit activations are one fp16 number, fp32 ones two (x = x1 + x2, as the decode
-// kernels split them): one or two tcgen05 products per term.  The products of one quantisation group -- 64 codes, or 32
+// instructions per pair of codes.  fp16 activations are the B operand as they are; bf16 and fp32 ones are scaled by a
+// power of two per token first, which the stored outputs undo, and are then one fp16 number and two (x = x1 + x2): one or
+// two tcgen05 products per term.  The products of one quantisation group -- 64 codes, or 32
 // where the group is that short -- accumulate in fp32 in tensor memory; then every thread adds
 // scale * sum + (bias + scale * 2^(bits-1)) * (sum of the group's activations) to fp32 accumulators in its registers.
 // (Folding scale and bias into an A operand of two fp16 numbers needs no such drain, but tcgen05 cuts every sum off
@@ -92,6 +93,7 @@ struct ExactArgs {
     unsigned* err;
     const float2* table;        // [group][o_pad] (scale, bias + scale * 2^(bits-1))
     const float* xsum;          // [drain step][t_pad] sums of the activations
+    const float* unscale;       // [t_pad] the inverse of each token's power of two
     float* partial;             // [tile][segment][token][row of the tile] (S > 1)
     unsigned* counters;         // [tile][draining warp] (S > 1)
     long long y_stride;
@@ -366,6 +368,7 @@ qgemm_exact_kernel(const __grid_constant__ CUtensorMap map_x, const ExactArgs a)
             const int m_tile = u % a.m_tiles, seg = seg_of(u);
             const int trow = quad * 32 + lane, row = m_tile * BM + trow;
             const int n_tile = u / (a.m_tiles * a.S), tok0 = n_tile * BN + par * NC;
+            const float unscale = lane < NC ? __ldcg(a.unscale + tok0 + lane) : 0.0f;     // lane c: token c of this warp's
             uint64_t acc[NC / 2];
 #pragma unroll
             for (int i = 0; i < NC / 2; i++) acc[i] = 0ull;
@@ -404,7 +407,8 @@ qgemm_exact_kernel(const __grid_constant__ CUtensorMap map_x, const ExactArgs a)
             const float rb = (a.bias != nullptr && row < a.O) ? load_scalar(a.bias, a.bias_dtype, row) : 0.0f;
             auto store = [&](int c, float v) {
                 const int tok = tok0 + c;
-                if (row < a.O && tok < a.T) store_scalar(a.y, a.y_dtype, static_cast<size_t>(tok) * a.y_stride + row, v + rb);
+                const float u = __shfl_sync(0xffffffffu, unscale, c);
+                if (row < a.O && tok < a.T) store_scalar(a.y, a.y_dtype, static_cast<size_t>(tok) * a.y_stride + row, fmaf(v, u, rb));
             };
             if (a.S == 1) {
 #pragma unroll
@@ -463,44 +467,99 @@ qgemm_exact_kernel(const __grid_constant__ CUtensorMap map_x, const ExactArgs a)
 struct ExactStage {
     const void* x; int x_dtype; long long x_stride; __half* xs; int T, K, xs_parts, permuted;
     float* xsum; int t_pad, step_chunks;     // chunks of eight activations per drain step: 8 or 4
+    float* unscale;                          // [t_pad] what a token's outputs are multiplied by
     const void* s; const void* b; int s_dtype; int s_vec; int O, o_pad, groups; float centre; float2* table;
     unsigned* counters; int n_counters;
     unsigned x_blocks;
 };
 
-__global__ void __launch_bounds__(256) exact_stage_kernel(const ExactStage g) {
+// A token's power of two: its largest magnitude comes to [2^14, 2^15), so that no activation overflows fp16 and the low
+// parts are no subnormal numbers wherever that matters (what is lost lies below 2^-40 of the largest).  Unscaled, an
+// activation of 1e5 became infinity, and fp32 ones of 1e-4 kept 13 of their 24 bits.  fp16 activations are what they
+// are: factor one, as for a row with an infinity.
+__device__ __forceinline__ uint32_t scale_exponent(float largest) {
+    const uint32_t e = __float_as_uint(largest) >> 23;                        // (sign bit clear)
+    return e == 255u ? 127u : min(268u - e, 253u);                            // biased; the inverse is 254 - it, never subnormal
+}
+
+constexpr int STAGE_THREADS = 256;
+constexpr int STAGE_KEEP = 6;                // chunks of a thread that stay in registers between the two passes: 12288 codes
+
+__global__ void __launch_bounds__(STAGE_THREADS) exact_stage_kernel(const ExactStage g) {
     if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");           // a dependent of the previous kernel; what that wrote is read through L2
     if (blockIdx.x < g.x_blocks) {
+        // a block per token: the largest magnitude first, then the parts
+        __shared__ float warp_max[STAGE_THREADS / 32];
         const int chunks = g.K / 8;                              // a multiple of 16
-        const long long n = static_cast<long long>(g.T) * chunks;
-        // (whole warps stay in the loop together: n is a multiple of 16, the sums are formed by 4 or 8 lanes)
-        for (long long i0 = blockIdx.x * 256ll + (threadIdx.x & ~31); i0 < n; i0 += g.x_blocks * 256ll) {
-            const long long i = i0 + (threadIdx.x & 31);
-            const bool live = i < n;
-            const int t = live ? static_cast<int>(i / chunks) : 0, c = live ? static_cast<int>(i - static_cast<long long>(t) * chunks) : 0;
-            const size_t at = static_cast<size_t>(t) * g.x_stride + c * 8;
-            float v[8];
-            load8_coherent(g.x, g.x_dtype, at, v);
-            float sum = 0.0f;
+        const int lane = threadIdx.x & 31;
+        for (int t = blockIdx.x; t < g.T; t += g.x_blocks) {
+            const size_t row = static_cast<size_t>(t) * g.x_stride;
+            float kept[STAGE_KEEP][8], largest = 0.0f;
 #pragma unroll
-            for (int j = 0; j < 8; j++) sum += v[j];
-            uint32_t hi[4], lo[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const float p = g.permuted ? v[j] : v[2 * j], q = g.permuted ? v[j + 4] : v[2 * j + 1];
-                const __half2 h = __floats2half2_rn(p, q);
-                const float2 f = __half22float2(h);
-                const __half2 l = __floats2half2_rn(p - f.x, q - f.y);
-                hi[j] = *reinterpret_cast<const uint32_t*>(&h);
-                lo[j] = *reinterpret_cast<const uint32_t*>(&l);
+            for (int k = 0; k < STAGE_KEEP; k++) {
+                const int c = k * STAGE_THREADS + threadIdx.x;
+                if (c < chunks) load8_coherent(g.x, g.x_dtype, row + c * 8, kept[k]);
             }
-            for (int o = 1; o < g.step_chunks; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            if (!live) continue;
-            __half* out = g.xs + static_cast<size_t>(t) * g.K + c * 8;
-            *reinterpret_cast<uint4*>(out) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            if (g.xs_parts == 2) *reinterpret_cast<uint4*>(out + static_cast<size_t>(g.T) * g.K) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-            if ((c & (g.step_chunks - 1)) == 0) g.xsum[static_cast<size_t>(c / g.step_chunks) * g.t_pad + t] = sum;
+            float factor = 1.0f, inverse = 1.0f;
+            if (g.x_dtype != DT_F16) {
+#pragma unroll
+                for (int k = 0; k < STAGE_KEEP; k++)
+                    if (k * STAGE_THREADS + static_cast<int>(threadIdx.x) < chunks)
+#pragma unroll
+                        for (int j = 0; j < 8; j++) largest = fmaxf(largest, fabsf(kept[k][j]));
+                for (int c = STAGE_KEEP * STAGE_THREADS + threadIdx.x; c < chunks; c += STAGE_THREADS) {
+                    float v[8];
+                    load8_coherent(g.x, g.x_dtype, row + c * 8, v);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) largest = fmaxf(largest, fabsf(v[j]));
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, o));
+                __syncthreads();                                 // (the previous token's maxima have been read)
+                if (lane == 0) warp_max[threadIdx.x >> 5] = largest;
+                __syncthreads();
+#pragma unroll
+                for (int w = 0; w < STAGE_THREADS / 32; w++) largest = fmaxf(largest, warp_max[w]);
+                const uint32_t e = scale_exponent(largest);
+                factor = __uint_as_float(e << 23);
+                inverse = __uint_as_float((254u - e) << 23);
+            }
+            if (threadIdx.x == 0) g.unscale[t] = inverse;
+            // one chunk of eight; whole warps come here together: the sums are formed by 4 or 8 lanes, which are live together
+            auto emit = [&](int c, const float (&v)[8], bool live) {
+                float sum = 0.0f, f[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) { f[j] = v[j] * factor; sum += f[j]; }
+                for (int o = 1; o < g.step_chunks; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                if (!live) return;
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float p = g.permuted ? f[j] : f[2 * j], q = g.permuted ? f[j + 4] : f[2 * j + 1];
+                    const __half2 h = __floats2half2_rn(p, q);
+                    const float2 b = __half22float2(h);
+                    const __half2 l = __floats2half2_rn(p - b.x, q - b.y);
+                    hi[j] = *reinterpret_cast<const uint32_t*>(&h);
+                    lo[j] = *reinterpret_cast<const uint32_t*>(&l);
+                }
+                __half* out = g.xs + static_cast<size_t>(t) * g.K + c * 8;
+                *reinterpret_cast<uint4*>(out) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                if (g.xs_parts == 2) *reinterpret_cast<uint4*>(out + static_cast<size_t>(g.T) * g.K) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                if ((c & (g.step_chunks - 1)) == 0) g.xsum[static_cast<size_t>(c / g.step_chunks) * g.t_pad + t] = sum;
+            };
+#pragma unroll
+            for (int k = 0; k < STAGE_KEEP; k++)
+                if (k * STAGE_THREADS < chunks) {
+                    const int c = k * STAGE_THREADS + threadIdx.x;
+                    emit(c, kept[k], c < chunks);
+                }
+            for (int c0 = STAGE_KEEP * STAGE_THREADS; c0 < chunks; c0 += STAGE_THREADS) {
+                const int c = c0 + threadIdx.x;
+                float v[8] = {};
+                if (c < chunks) load8_coherent(g.x, g.x_dtype, row + c * 8, v);
+                emit(c, v, c < chunks);
+            }
         }
         return;
     }
@@ -635,13 +694,13 @@ cudaError_t launch_qgemm_exact(const GemmLayer& L, const GemmCall& c, cudaStream
     const long long n_tiles = (slice + bn - 1) / bn;
     a.t_pad = static_cast<int>(n_tiles) * bn;
     const size_t x_b = align256(static_cast<size_t>(slice) * L.K * 2 * parts), tab_b = align256(static_cast<size_t>(groups) * o_pad * sizeof(float2));
-    const size_t sum_b = align256(static_cast<size_t>(steps) * a.t_pad * 4);
+    const size_t sum_b = align256(static_cast<size_t>(steps) * a.t_pad * 4), un_b = align256(static_cast<size_t>(a.t_pad) * 4);
     const size_t ctr_b = a.S > 1 ? align256(static_cast<size_t>(n_tiles) * a.m_tiles * WORKERS * 4) : 0;
     const size_t part_b = a.S > 1 ? static_cast<size_t>(n_tiles) * a.m_tiles * a.S * bn * BM * 4 : 0;
     cudaMemPool_t pool = gemm_scratch_pool(L.device);
     if (!pool) { *why = "scratch pool"; return cudaErrorMemoryAllocation; }
     uint8_t* scratch = nullptr;
-    if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch), x_b + tab_b + sum_b + ctr_b + part_b, pool, st) != cudaSuccess) {
+    if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch), x_b + tab_b + sum_b + un_b + ctr_b + part_b, pool, st) != cudaSuccess) {
         cudaGetLastError();
         *why = "scratch allocation";
         return cudaErrorMemoryAllocation;
@@ -651,8 +710,10 @@ cudaError_t launch_qgemm_exact(const GemmLayer& L, const GemmCall& c, cudaStream
     float* xsum = reinterpret_cast<float*>(scratch + x_b + tab_b);
     a.table = table;
     a.xsum = xsum;
-    a.counters = reinterpret_cast<unsigned*>(scratch + x_b + tab_b + sum_b);
-    a.partial = reinterpret_cast<float*>(scratch + x_b + tab_b + sum_b + ctr_b);
+    float* unscale = reinterpret_cast<float*>(scratch + x_b + tab_b + sum_b);
+    a.unscale = unscale;
+    a.counters = reinterpret_cast<unsigned*>(scratch + x_b + tab_b + sum_b + un_b);
+    a.partial = reinterpret_cast<float*>(scratch + x_b + tab_b + sum_b + un_b + ctr_b);
     // fp32 accumulate, A and B fp16, both K-major, N = bn, M = 128
     a.idesc = (1u << 4) | (static_cast<uint32_t>(bn >> 3) << 17) | (static_cast<uint32_t>(BM >> 4) << 24);
     cudaError_t err = cudaSuccess;
@@ -664,17 +725,16 @@ cudaError_t launch_qgemm_exact(const GemmLayer& L, const GemmCall& c, cudaStream
         ExactStage g = {};
         g.x = static_cast<const char*>(c.x) + static_cast<size_t>(t0) * c.x_stride * dtype_size(c.x_dtype);
         g.x_dtype = c.x_dtype; g.x_stride = c.x_stride; g.xs = xs; g.T = T; g.K = L.K; g.xs_parts = parts; g.permuted = L.bits == 4;
-        g.xsum = xsum; g.t_pad = a.t_pad; g.step_chunks = 8 >> a.steps_shift;
+        g.xsum = xsum; g.unscale = unscale; g.t_pad = a.t_pad; g.step_chunks = 8 >> a.steps_shift;
         g.s = L.s; g.b = L.b; g.s_dtype = L.s_dtype; g.O = L.O; g.o_pad = o_pad; g.groups = groups;
         g.s_vec = groups % 8 == 0 && ((reinterpret_cast<uintptr_t>(L.s) | reinterpret_cast<uintptr_t>(L.b)) & 15u) == 0;
         g.centre = static_cast<float>(1 << (L.bits - 1)); g.table = table;
         g.counters = a.counters; g.n_counters = a.S > 1 ? a.n_tiles * a.m_tiles * WORKERS : 0;
-        const long long nx = (static_cast<long long>(T) * (L.K / 8) + 255) / 256;
         const long long ns = (static_cast<long long>((groups + 7) / 8) * o_pad + 255) / 256;
-        g.x_blocks = static_cast<unsigned>(nx < 148 * 6 ? nx : 148 * 6);
+        g.x_blocks = static_cast<unsigned>(T < 148 * 6 ? T : 148 * 6);
         cudaLaunchConfig_t sc = {};
         sc.gridDim = dim3(g.x_blocks + static_cast<unsigned>(ns < 148 * 4 ? ns : 148 * 4));
-        sc.blockDim = dim3(256);
+        sc.blockDim = dim3(STAGE_THREADS);
         sc.stream = st;
         cudaLaunchAttribute sa[1];
         sa[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -242,3 +242,38 @@ def test_captured_long_batches_need_no_allocation_nodes(mlxq, oracle):
     torch.cuda.synchronize()
     mlxq.streamStatus(None, 0)
     assert float(np.linalg.norm(y.cpu().numpy() - eager) / np.linalg.norm(eager)) < 5e-6
+
+
+@pytest.mark.parametrize("bits,gs,K,O", [(8, 64, 12288, 40), (4, 64, 12288, 24), (2, 32, 256, 40), (6, 128, 14336, 24)])
+@pytest.mark.parametrize("x_dtype", [0, 2])
+def test_full_precision_gemm_at_any_magnitude(mlxq, oracle, bits, gs, K, O, x_dtype):
+    # activations outside fp16's range: tokens of 1e-38 ... 1e30, one whose elements span ten orders of magnitude, one of
+    # zeros, and next to them one with an infinity.  A token's power of two leaves what lies above 2^-40 of its largest
+    # element as exact as at magnitude one, so every token meets the same bar as there (1e-6 of its norm).
+    if bits == 4 and x_dtype != 0:
+        x_dtype = 0                                                # (16-bit activations on 4-bit layers take the other GEMM)
+    fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=gs, scale_type=oracle.BF16, seed=bits + K)
+    layer = DevLayer.from_fixture(mlxq, fx)
+    mags = [1e-38, 1e-20, 1e-5, 1e-4, 1e-3, 1e-2, 1.0, 1e2, 7e4, 1e5, 1e10, 1e30]
+    T = len(mags) + 8
+    x = oracle.RNG(K + bits).floats(T * K).reshape(T, K)
+    for t, m in enumerate(mags):
+        x[t] = (x[t].astype(np.float64) * m).astype(np.float32)
+    n = len(mags)
+    x[n] = (x[n] * np.exp(np.linspace(0.0, 23.0, K))).astype(np.float32)
+    x[n + 1] = 0.0
+    x[n + 2, 5] = np.inf
+    xr = as_dtype(x, x_dtype).float().cpu().numpy()
+    got = run(layer, x, T, x_dtype=x_dtype).astype(np.float64)
+    mlxq.streamStatus(None, 0)
+    finite = [t for t in range(T) if t != n + 2]
+    w = np.repeat(oracle.to_float(fx.scales_raw, oracle.BF16), gs, axis=1).astype(np.float64) * fx.q + \
+        np.repeat(oracle.to_float(fx.biases_raw, oracle.BF16), gs, axis=1).astype(np.float64)
+    ref = xr[finite].astype(np.float64) @ w.T
+    for i, t in enumerate(finite):
+        if t == n + 1:
+            assert not got[t].any()
+            continue
+        err = float(np.linalg.norm(got[t] - ref[i]) / np.linalg.norm(ref[i]))
+        assert err < 1e-6, f"bits {bits} x dtype {x_dtype} token {t} (largest {np.abs(xr[t]).max():.3g}): {err}"
+    assert not np.isfinite(got[n + 2]).any()
