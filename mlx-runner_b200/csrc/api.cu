@@ -307,25 +307,40 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
         }
         PipePlan pp;
         const size_t rsmem = !persistent ? 0 : qmv_pipe_plan(parts[0]->bits, mp, static_cast<int>(T), device_sm_count(parts[0]->device), pp);
-        if (peer && !rsmem) return fail(MLXQ_UNSUPPORTED, "this shape does not run on the persistent decode kernel: no fused gather");
-        // does a call of `t` tokens run on one of the persistent kernels?
-        auto fits_persistent = [&](int64_t t) {
+        // does a call of `t` tokens run on one of the persistent kernels (2: on the token-major one)?
+        auto fits_persistent = [&](int64_t t) -> int {
             MmaParams m2;
             bool ok2 = false;
             mma_plan(parts, n, x_dtype, t, m2, &ok2);
-            if (!ok2) return false;
+            if (!ok2) return 0;
             m2.q = p;
             m2.q.T = static_cast<int>(t);
             m2.err = mp.err;
             TokPlan t2;
             PipePlan p2;
             const int sms = device_sm_count(parts[0]->device);
-            return (t >= 2 && qmv_tok_plan(parts[0]->bits, m2, static_cast<int>(t), sms, t2) != 0) || qmv_pipe_plan(parts[0]->bits, m2, static_cast<int>(t), sms, p2) != 0;
+            if (t >= 2 && qmv_tok_plan(parts[0]->bits, m2, static_cast<int>(t), sms, t2)) return 2;
+            return qmv_pipe_plan(parts[0]->bits, m2, static_cast<int>(t), sms, p2) ? 1 : 0;
         };
         const int64_t h0 = T / 2;
-        if (persistent && !rsmem && T >= 4 && fits_persistent(h0) && fits_persistent(T - h0)) {
-            // Too many staged activation columns for a CTA's shared memory (long rows): two calls of half the tokens,
-            // each on a persistent kernel, beat the register-fed kernel although the weights are read twice.
+        const int fit = persistent && !rsmem && T >= 4 ? fits_persistent(h0) * fits_persistent(T - h0) : 0;
+        if (persistent && !rsmem && T >= 2 && !(mode && strcmp(mode, "pipe") == 0) && (fit == 4 || peer || (x_up && !fit))) {
+            // Too many staged activation columns for a CTA's shared memory (long rows): the token-major kernel with K split
+            // over a cluster, in the place of two of its calls with half the tokens.  Not in the place of another kernel: the
+            // one-token kernel's sums are the more exact ones (8 bits, 4096 x 12288, 3 fp32 tokens: 2.0e-7 of the result
+            // against 5.5e-7), and the CUDA-core kernel multiplies in fp32, at any magnitude of the activations.
+            TokPlan tp;
+            const size_t tsmem = qmv_tok_plan(parts[0]->bits, mp, static_cast<int>(T), device_sm_count(parts[0]->device), tp, true);
+            if (tsmem) {
+                const cudaError_t err = launch_qmv_tok(parts[0]->bits, mp, tp, tsmem, parts[0]->device, st);
+                if (err != cudaSuccess) return cuda_fail(err, "qmv (token-major, cluster) launch");
+                return MLXQ_OK;
+            }
+        }
+        if (peer && !rsmem) return fail(MLXQ_UNSUPPORTED, "this shape does not run on the persistent decode kernel: no fused gather");
+        if (fit) {
+            // ... or two calls of half the tokens: each on a persistent kernel, they beat the register-fed kernel although
+            // the weights are read twice.
             const int rc = run_qmv(parts, n, st, x, x_dtype, x_stride, y, y_dtype, y_stride, h0, e, act, nullptr, x_up, x_act);
             if (rc != MLXQ_OK) return rc;
             return run_qmv(parts, n, st, static_cast<const char*>(x) + static_cast<size_t>(h0) * x_stride * dtype_size(x_dtype), x_dtype, x_stride,

@@ -120,16 +120,14 @@ int cluster_capacity(int kz, int sms) {
     return cached[dev][slot];
 }
 
-// CTAs that share K, from the layer alone, so that a token's sums do not change with the batch.  Measured with 1 / 2 / 4 / 8
-// CTAs, fp32 tokens: 4096 x 12288 with 6 tokens 27.8 / 27.6 / 25.1 / 24.1 us (45.7 on the one-token kernel, which long rows
-// fell back to; 8 bits 124 -> 20.8), 2048 x 6144 with 4 tokens 11.3 / 9.7 / 9.0 / 9.3; but 4096 x 4096 with 2 tokens
-// 8.1 / 8.5 / 8.9 / 11.3, and 28672 x 8192 63.1 / 63.0 / 66.1 / 73.7: with many blocks the clusters that a part of the chip
+// CTAs that share K where they do, doubled until the tokens fit.  Measured with 2 / 4 / 8 CTAs, fp32 tokens: 4096 x 12288
+// with 6 tokens 27.6 / 25.1 / 24.1 us; 28672 x 8192 63.0 / 66.1 / 73.7: with many blocks the clusters that a part of the chip
 // has no room for cost more than the shorter staging gives.
-int k_split(int K, int n_blocks) { return K >= 6144 && n_blocks <= 1024 ? 4 : 1; }
+int k_split(int n_blocks) { return n_blocks <= 1024 ? 4 : 2; }
 
 }  // namespace
 
-size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& tp) {
+size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& tp, bool clusters) {
     const QmvParams& q = p.q;
     if (tokens < 1 || q.total_rows < 1 || p.xn < 1 || p.xn > 16) return 0;
     if (q.gs != 32 && q.gs != 64 && q.gs != 128) return 0;
@@ -153,7 +151,7 @@ size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& 
     long long best_cost = -1;
     size_t best_total = 0;
     // (a split whose slices still do not fit a CTA's shared memory is doubled)
-    for (tp.kz = k_split(K, tp.n_blocks); tp.kz <= 8; tp.kz *= 2) {
+    for (tp.kz = clusters ? k_split(tp.n_blocks) : 1; tp.kz <= (clusters ? 8 : 1); tp.kz *= 2) {
         const int kz = tp.kz;
         if (groups / 2 < kz) break;
         const int room = kz == 1 ? sms : cluster_capacity(kz, sms), n_cl = tp.n_blocks < room ? tp.n_blocks : room;

@@ -16,11 +16,11 @@
 // else (warp-private cp.async rings, K split over `ks` warps with a named barrier per group of warps, dependent
 // launch, the peers' stores of sharded calls) is as in qmv_pipe.cuh.
 //
-// Long rows: K is also split over the `kz` CTAs of a thread-block cluster.  Each CTA stages only its slice of the
-// activations -- with all of K a CTA's shared memory holds 8 tokens of 12288, 4 in fp32, and the call fell back to two
-// calls of half the tokens on the one-token kernel -- and multiplies that slice of the cluster's blocks; the blocks' sums
-// stay in shared memory until the end, one cluster barrier later every CTA adds up and stores a share of them, reading the
-// others' through distributed shared memory in the order of the slices.
+// Long rows: where a CTA's shared memory does not hold all of K of the batch, K is also split over the `kz` CTAs of a
+// thread-block cluster (instead of two calls of half the tokens).  Each CTA stages only its slice of the activations and
+// multiplies that slice of the cluster's blocks; the blocks' sums stay in shared memory until the end, one cluster barrier
+// later every CTA adds up and stores a share of them, reading the others' through distributed shared memory in the order of
+// the slices.
 #pragma once
 
 #include "qmv_pipe.cuh"
@@ -553,7 +553,8 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
 }
 
 // Plans a call of the token-major kernel; returns the shared memory it needs, 0 when the call is not one it serves.
-size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& tp);
+// `clusters`: a plan with K split over the CTAs of a cluster, or else one for single CTAs.
+size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& tp, bool clusters = false);
 cudaError_t launch_qmv_tok(int bits, const MmaParams& p, const TokPlan& tp, size_t smem, int device, cudaStream_t st);
 
 }  // namespace mlxq

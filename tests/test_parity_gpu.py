@@ -195,6 +195,44 @@ def test_small_batches_of_long_rows(mlxq, oracle, bits):
         close(oracle, got, fx.reference(xr), f"bits {bits} gs {gs} {O}x{K} T {T} x {x_dtype}", (1e-4 if x_dtype == 0 else 3e-5) * (K / 1536) ** 0.5)
 
 
+@pytest.mark.parametrize("x_dtype,T", [(0, 9), (0, 16), (2, 16), (0, 24), (2, 24)])
+def test_batches_beyond_the_persistent_kernels_keep_fp32_products(mlxq, oracle, x_dtype, T):
+    # calls that no persistent kernel holds on single CTAs, as one call or as two halves, multiply in fp32: activations of
+    # 1e5, which an fp16 operand cannot hold, and of 1e-5, which it holds to a few bits.  24 tokens: the paths without
+    # scratch memory (static, captured, three layers in one launch).  The bar: fp32 sums of 14336 terms in 32 lanes, each
+    # rounding 448 times (2^-24 * sqrt(448 / 3) = 7e-7 of the result; measured 3e-7).
+    K, O, bits, gs = 14336, 24, 8, 64
+    fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=gs, scale_type=oracle.BF16, seed=T)
+    layer = DevLayer.from_fixture(mlxq, fx)
+    for mag in (1e5, 1e-5):
+        x = oracle.RNG(T).floats(T * K).reshape(T, K) * np.float32(mag)
+        xd = as_dtype(x, x_dtype)
+        ref = oracle.qmatmul(fx.packed, fx.scales_raw, fx.biases_raw, oracle.BF16, xd.float().cpu().numpy(), K, bits, gs)
+
+        def check(y, what):
+            torch.cuda.synchronize()
+            got = y.cpu().numpy()[:, :O]
+            nrm = float(np.linalg.norm(got - ref) / np.linalg.norm(ref))
+            assert nrm < 7e-7, f"{what}, x dtype {x_dtype}, {T} tokens of {mag:g}: {nrm}"
+
+        y = torch.full((T, O), float("nan"), device="cuda")
+        if T <= 16:
+            layer.linear.encode(None, xd, K, y, O, T)
+            check(y, "forward")
+            continue
+        layer.linear.encodeStatic(None, xd, K, y, O, T)
+        check(y, "static")
+        y.fill_(float("nan"))
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            layer.linear.encode(torch.cuda.current_stream(), xd, K, y, O, T)
+        g.replay()
+        check(y, "captured")
+        y3 = torch.full((T, 3 * O), float("nan"), device="cuda")
+        mlxq.Linear.encodeFusedDecode(None, [layer.linear] * 3, xd, y3, xStride=K, yStride=3 * O, T=T)
+        check(y3, "fused")
+
+
 @pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
 def test_one_fp32_token_every_width_and_group(mlxq, oracle, bits):
     # one fp32 token: its two fp16 parts on the kernel compiled for the group size, where slices of K hold whole drain
