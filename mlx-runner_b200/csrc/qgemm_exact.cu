@@ -26,7 +26,7 @@
 //
 // Split K.  A layer of few rows leaves most SMs without a tile, so K is cut into `S` segments worked on by different
 // CTAs; the warp that finishes a piece of the tile last adds the segments' partial sums in their order.  S depends on
-// the layer alone, not on the batch: a token's result is the same whatever batch it rides in.
+// the layer and the activations' type alone, not on the batch: a token's result is the same whatever batch it rides in.
 // Measured (pre-pass included, one decode-kernel pass per eight tokens before): 12288 x 4096, 4 bits, 512 fp32 tokens
 // 1398 -> 165 us (312 TFLOP/s counted once per term); 8 bits, 384 bf16 tokens 717 -> 121 us.  What bounds it now is the
 // drain: 128 x 128 sums leave tensor memory per 64 codes, two packed FMAs per pair of them, some 1700 cycles a stage
@@ -645,18 +645,29 @@ cudaError_t launch_bits(int bits, int bn, const CUtensorMap& map_x, const ExactA
 size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 
 // Segments of K: the count that leaves the busiest CTA the least to do on one tile of tokens, from the layer alone (a
-// unit's fixed cost is about six stages; a segment keeps eight stages or more).  Never from the device or the batch:
-// the order of the sums must not change with them.
-int segments(int m_tiles, int k_stages) {
+// unit's fixed cost is about six stages; a segment keeps eight stages or more), but no fewer than `least`.  Never from the
+// device or the batch: the order of the sums must not change with them.
+int segments(int m_tiles, int k_stages, int least) {
     constexpr int SMS = 148;
-    int best = 1;
+    int best = least;
     long long best_cost = -1;
-    for (int s = 1; s <= 8 && (s == 1 || k_stages / s >= 8); s++) {
+    for (int s = least; s == least || (s <= 8 && k_stages / s >= 8); s++) {
         const long long waves = (static_cast<long long>(m_tiles) * s + SMS - 1) / SMS;
         const long long cost = waves * ((k_stages + s - 1) / s + 6);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
     }
     return best;
+}
+
+// 8-bit rows of more than 8192 codes with 16-bit activations, which the CUDA-core kernel serves otherwise: segments of 24
+// drain steps at most, 16 of them at most, so that the error is not above that kernel's.  The products are exact here and
+// the roundings of the running sum are what is left; in sums of 48 and 96 steps they came to 1.34e-7 and 1.82e-7 of the
+// result (12288 codes in groups of 64 and 32), in sums of 24 to 1.1e-7 and 1.2e-7, there to 1.2e-7.  (4096 x 12288 with 384
+// bf16 tokens: 129 -> 141 us in groups of 64, 209 -> 260 in groups of 32.)
+int least_segments(const GemmLayer& L, int parts) {
+    if (L.bits != 8 || parts != 1 || L.K <= 8192) return 1;
+    const int steps = L.K / (L.gs == 32 ? 32 : BK), s = (steps + 23) / 24;
+    return s < 16 ? s : 16;
 }
 
 constexpr long long SLICE_BYTES = 96ll << 20;          // scratch of one slice of tokens, about
@@ -683,7 +694,7 @@ cudaError_t launch_qgemm_exact(const GemmLayer& L, const GemmCall& c, cudaStream
     while ((1 << a.gs_shift) < L.gs) a.gs_shift++;
     a.steps_shift = L.gs == 32 ? 1 : 0;
     a.m_tiles = (L.O + BM - 1) / BM;
-    a.S = segments(a.m_tiles, L.K / BK);
+    a.S = segments(a.m_tiles, L.K / BK, least_segments(L, parts));
     const int steps = (L.K / BK) << a.steps_shift, groups = L.K / L.gs, o_pad = a.m_tiles * BM;
     // Long batches run in slices of tokens, so that the scratch memory stays bounded whatever the batch.
     const long long per_token = static_cast<long long>(L.K) * 2 * parts + 4ll * steps + (a.S > 1 ? 4ll * a.S * o_pad : 0);

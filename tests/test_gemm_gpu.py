@@ -277,3 +277,27 @@ def test_full_precision_gemm_at_any_magnitude(mlxq, oracle, bits, gs, K, O, x_dt
         err = float(np.linalg.norm(got[t] - ref[i]) / np.linalg.norm(ref[i]))
         assert err < 1e-6, f"bits {bits} x dtype {x_dtype} token {t} (largest {np.abs(xr[t]).max():.3g}): {err}"
     assert not np.isfinite(got[n + 2]).any()
+
+
+@pytest.mark.parametrize("gs", [32, 64])
+def test_full_precision_gemm_on_long_8_bit_rows(mlxq, oracle, gs):
+    # rows beyond 8192 codes on a layer with a row tile for every SM, where K would otherwise be one sum of 132 (264) steps.
+    # Rounding 24 times a running sum that grows like their square root: 2^-24 * sqrt(24 / 2) / sqrt(3) = 1.2e-7 of the result;
+    # the tensor core drops up to 2^-25 of a group's sum at each of its four steps, half of it on average: 0.6e-7.
+    # Together 1.4e-7; one sum gives 2.0e-7 and 2.9e-7.
+    O, K, T = 18944, 8448, 20
+    rng = np.random.default_rng(gs)
+    q = rng.integers(0, 256, (O, K), dtype=np.uint8)
+    s = torch.from_numpy((np.abs(rng.standard_normal((O, K // gs))) * 0.002 + 1e-4).astype(np.float32)).to(torch.bfloat16)
+    b = (-128.0 * s.float()).to(torch.bfloat16)
+    x = torch.from_numpy(rng.standard_normal((T, K)).astype(np.float32)).to(torch.bfloat16)
+    lin = mlxq.Linear(torch.from_numpy(q.view(np.int32)).cuda(), s.cuda(), b.cuda(), None, inDim=K)
+    y = torch.full((T, O), float("nan"), device="cuda")
+    lin.encode(None, x.cuda(), K, y, O, T)
+    torch.cuda.synchronize()
+    mlxq.streamStatus(None, 0)
+    rows = rng.choice(O, 96, replace=False)
+    w = np.repeat(s.double().numpy()[rows], gs, axis=1) * q[rows] + np.repeat(b.double().numpy()[rows], gs, axis=1)
+    ref = x.double().numpy() @ w.T
+    nrm = float(np.linalg.norm(y.cpu().numpy()[:, rows] - ref) / np.linalg.norm(ref))
+    assert nrm < 1.4e-7, f"gs {gs}: normwise {nrm}"
