@@ -10,7 +10,7 @@
 // it (with six tokens the step took 4770 us, with the chain 4326).
 #include "aux_kernels.cuh"
 
-#include <cstdlib>
+#include "dependent_launch.h"
 
 namespace mlxq {
 
@@ -22,7 +22,6 @@ __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontr
 // Launches `kernel` as a programmatic dependent of the stream's previous kernel (MLXQ_PDL=0: as an ordinary one).
 template <class... P, class... A>
 cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
-    static const bool pdl = [] { const char* e = std::getenv("MLXQ_PDL"); return !(e && e[0] == '0'); }();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -31,7 +30,7 @@ cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaSt
     la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     la[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = la;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 

@@ -39,6 +39,7 @@
 
 #include <mutex>
 
+#include "dependent_launch.h"
 #include "mlxq_device.cuh"
 #include "qgemm_exact.cuh"
 #include "qmv_pipe.cuh"
@@ -199,7 +200,7 @@ qgemm_exact_kernel(const __grid_constant__ CUtensorMap map_x, const ExactArgs a)
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base), 0);
 
-    // (the packed weights are the layer's constants: the unpacking warps do not wait for the pre-pass)
+    // (the unpacking warps do not wait for the pre-pass, which lets this grid start when all before it is complete)
     if (warp >= WORKER0) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (warp == X_PRODUCER) {
         if (lane == 0) {
@@ -486,8 +487,10 @@ constexpr int STAGE_THREADS = 256;
 constexpr int STAGE_KEEP = 6;                // chunks of a thread that stay in registers between the two passes: 12288 codes
 
 __global__ void __launch_bounds__(STAGE_THREADS) exact_stage_kernel(const ExactStage g) {
-    if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");           // a dependent of the previous kernel; what that wrote is read through L2
+    // The GEMM may start now and not before: it reads packed weights without a wait of its own, and everything ahead in the
+    // stream, which may have written them, is complete here.
+    if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (blockIdx.x < g.x_blocks) {
         // a block per token: the largest magnitude first, then the parts
         __shared__ float warp_max[STAGE_THREADS / 32];
@@ -618,7 +621,7 @@ cudaError_t launch_one(const CUtensorMap& map_x, const ExactArgs& a, int device,
     la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;          // a dependent of the pre-pass
     la[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = la;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, qgemm_exact_kernel<BITS, XS, NC>, map_x, a);
 }
 
@@ -751,7 +754,7 @@ cudaError_t launch_qgemm_exact(const GemmLayer& L, const GemmCall& c, cudaStream
         sa[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         sa[0].val.programmaticStreamSerializationAllowed = 1;
         sc.attrs = sa;
-        sc.numAttrs = 1;
+        sc.numAttrs = pdl_enabled() ? 1 : 0;
         err = cudaLaunchKernelEx(&sc, exact_stage_kernel, g);
         if (err != cudaSuccess) { *why = "pre-pass"; break; }
         CUtensorMap map_x;

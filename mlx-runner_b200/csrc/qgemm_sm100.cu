@@ -39,6 +39,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "dependent_launch.h"
 #include "mlxq_device.cuh"
 #include "qgemm.cuh"
 #include "sm100_ptx.cuh"
@@ -785,11 +786,12 @@ struct StageArgs {
     unsigned x_blocks;
 };
 __global__ void stage_inputs_kernel(const StageArgs g) {
-    // the GEMM that follows is launched as a programmatic dependent: it may set up (barriers, tensor memory, first
-    // weight slabs) while this grid runs, and waits for this grid before it touches what is written here
-    if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // ... and is itself a dependent of the stream's previous kernel: it neither reads nor writes anything before that is done
+    // a dependent of the stream's previous kernel: it neither reads nor writes anything before that is done
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    // The GEMM that follows is a programmatic dependent of this grid: it may set up (barriers, tensor memory, first weight
+    // slabs) while this grid runs, and waits for it before it touches what is written here.  It is let go only now that
+    // everything ahead in the stream is complete, since that may have written the packed weights.
+    if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (blockIdx.x < g.x_blocks) stage_x_part(g.x, g.is_bf16, g.x_stride, g.xs, g.T, g.K, blockIdx.x, g.x_blocks);
     else stage_scales_part(g.s, g.b, g.s_dtype, g.O, g.o_pad, g.gpr, g.gs_shift, g.k_stages, g.n_slabs, g.pairs,
                            blockIdx.x - g.x_blocks, gridDim.x - g.x_blocks);
@@ -953,7 +955,7 @@ cudaError_t enqueue_gemm(const GemmLayer& L, const GemmCall& c, cudaStream_t st,
         sa[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         sa[0].val.programmaticStreamSerializationAllowed = 1;
         sc.attrs = sa;
-        sc.numAttrs = 1;
+        sc.numAttrs = pdl_enabled() ? 1 : 0;
         const cudaError_t se = cudaLaunchKernelEx(&sc, stage_inputs_kernel, g);
         if (se != cudaSuccess) { *why = "pre-pass"; return se; }
     }
@@ -982,7 +984,7 @@ cudaError_t enqueue_gemm(const GemmLayer& L, const GemmCall& c, cudaStream_t st,
     la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;       // a dependent of the pre-pass, see the kernels
     la[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = la;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
     if (wide_tile) return cudaLaunchKernelEx(&cfg, wide::qgemm4w_kernel<256>, map_w, map_x, a);
     if (!tall) return cudaLaunchKernelEx(&cfg, wide::qgemm4w_kernel<128>, map_w, map_x, a);
     return cudaLaunchKernelEx(&cfg, qgemm4_kernel, map_w, map_x, a);

@@ -1,5 +1,6 @@
 // Planner, instantiations and launcher of the persistent decode matvec fed by warp-private asynchronous copies
 // (qmv_pipe.cuh).
+#include "dependent_launch.h"
 #include "qmv_pipe.cuh"
 
 #include <cstdlib>
@@ -25,12 +26,6 @@ void unit_for(int bits, int& lb, int& kb) {
 }
 
 int align_up(int v, int a) { return (v + a - 1) / a * a; }
-
-// MLXQ_PDL=0 launches without the programmatic-dependent-launch attribute (see the kernel's prologue).
-bool pdl_enabled() {
-    static const bool v = [] { const char* e = std::getenv("MLXQ_PDL"); return !(e && e[0] == '0'); }();
-    return v;
-}
 
 template <int BITS, int NP, int UNR, int GS, int SPX>
 cudaError_t launch_one(const MmaParams& p, const PipePlan& pp, size_t smem, int device, cudaStream_t st) {

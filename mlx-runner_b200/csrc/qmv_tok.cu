@@ -1,4 +1,5 @@
 // Planner, instantiations and launcher of the token-major decode matvec for small batches (qmv_tok.cuh).
+#include "dependent_launch.h"
 #include "qmv_tok.cuh"
 
 #include <cstdlib>
@@ -11,11 +12,6 @@ namespace {
 constexpr int SMEM_WHOLE = 224 * 1024;      // of the 227 KB a CTA may opt into
 
 int align_up(int v, int a) { return (v + a - 1) / a * a; }
-
-bool pdl_enabled() {
-    static const bool v = [] { const char* e = std::getenv("MLXQ_PDL"); return !(e && e[0] == '0'); }();
-    return v;
-}
 
 bool supported(int bits, int gs) {
     const int gb_bits = gs * bits;                  // bits of a group per row

@@ -301,3 +301,67 @@ def test_full_precision_gemm_on_long_8_bit_rows(mlxq, oracle, gs):
     ref = x.double().numpy() @ w.T
     nrm = float(np.linalg.norm(y.cpu().numpy()[:, rows] - ref) / np.linalg.norm(ref))
     assert nrm < 1.4e-7, f"gs {gs}: normwise {nrm}"
+
+
+@pytest.mark.parametrize("bits,x_dtype", [(4, 2), (8, 2), (4, 0)])
+def test_gemm_reads_weights_written_just_ahead_in_the_stream(mlxq, bits, x_dtype):
+    # A kernel of the library that lets its successor start early (the activation product) writes the packed weights; the
+    # GEMM behind it must see all of them.  (Its pre-pass is a dependent launch too, so nothing but its own order of wait and
+    # trigger keeps the GEMM from reading ahead.)
+    O, K, T = 4096, 4096, 64
+    words = O * K * bits // 32
+    cols, rows = 4096, words // 4096
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(bits)
+    w = torch.zeros(words, device="cuda")
+    gu = torch.randn((rows, 2 * cols), device="cuda", generator=gen)
+    s = (torch.rand((O, K // 64), device="cuda", generator=gen) * 0.01).to(torch.bfloat16)
+    lin = mlxq.Linear(w.view(torch.int32).view(O, -1), s, s.clone(), None, inDim=K)
+    lin.prepare()
+    x = torch.randn((T, K), device="cuda", generator=gen).to({0: torch.float32, 2: torch.bfloat16}[x_dtype])
+    y, ref = torch.zeros((T, O), device="cuda"), torch.zeros((T, O), device="cuda")
+    mlxq.actMul(None, gu, 2 * cols, cols, rows, mlxq.ACT_SILU, w)
+    torch.cuda.synchronize()
+    lin.encode(None, x, K, ref, O, T)
+    for _ in range(20):
+        w.zero_()
+        torch.cuda.synchronize()
+        mlxq.actMul(None, gu, 2 * cols, cols, rows, mlxq.ACT_SILU, w)
+        lin.encode(None, x, K, y, O, T)
+        torch.cuda.synchronize()
+        assert torch.equal(y, ref)
+    mlxq.streamStatus(None, 0)
+
+
+_ORDINARY_LAUNCHES = """
+import importlib, sys, torch
+mlxq, out = importlib.import_module("mlx-runner_b200"), {}
+gen = torch.Generator(device="cuda"); gen.manual_seed(3)
+for bits in (4, 8):
+    w = torch.randint(-(1 << 31), (1 << 31) - 1, (264, 512 * bits // 32), dtype=torch.int32, device="cuda", generator=gen)
+    s = torch.rand((264, 8), device="cuda", generator=gen).to(torch.bfloat16)
+    lin = mlxq.Linear(w, s, s.clone(), None, inDim=512)
+    for T in (1, 3, 20, 200):
+        x = torch.randn((T, 512), device="cuda", generator=gen).to(torch.bfloat16)
+        y = torch.zeros((T, 264), device="cuda")
+        lin.encode(None, x, 512, y, 264, T)
+        a = torch.zeros((T, 132), device="cuda")
+        mlxq.actMul(None, y, 264, 132, T, mlxq.ACT_SILU, a)
+        out[bits, T] = (y.cpu(), a.cpu())
+torch.save(out, sys.argv[1])
+"""
+
+
+def test_ordinary_launches_give_the_same_bits(mlxq, tmp_path):
+    # MLXQ_PDL=0 (read once per process, hence the child processes) turns every dependent launch into an ordinary one
+    import os
+    import subprocess
+    import sys
+    got = []
+    for v in ("0", "1"):
+        out = tmp_path / f"pdl{v}.pt"
+        subprocess.run([sys.executable, "-c", _ORDINARY_LAUNCHES, str(out)], check=True, timeout=300, env={**os.environ, "MLXQ_PDL": v},
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+        got.append(torch.load(out))
+    for key, (y, a) in got[0].items():
+        assert torch.equal(y, got[1][key][0]) and torch.equal(a, got[1][key][1]), key
