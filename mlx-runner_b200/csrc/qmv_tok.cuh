@@ -84,8 +84,9 @@ __device__ __forceinline__ void mma1688_tf32(float (&d)[4], uint32_t a0, uint32_
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// (not the .aligned form: the loops before it run a different number of turns in the lanes of a warp)
 __device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 // the float at shared address `addr` of CTA `rank` of the cluster
 __device__ __forceinline__ float cluster_load(uint32_t addr, int rank) {
@@ -527,6 +528,7 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
                 if (!CLUSTER || kz == 1) finish(c_blk * 16 + r, tok, v);
                 else zsum[((gi + bj * n_groups) * T + tok) * 16 + r] = v;
             }
+            __syncwarp();                                       // (an odd T leaves the half warps at different turns; what follows wants whole warps)
         }
         if (tp.parities == 1 && ks > 1) asm volatile("bar.sync %0, %1;" ::"r"(1 + gi), "r"(ks * 32) : "memory");
     }

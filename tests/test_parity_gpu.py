@@ -195,6 +195,25 @@ def test_small_batches_of_long_rows(mlxq, oracle, bits):
         close(oracle, got, fx.reference(xr), f"bits {bits} gs {gs} {O}x{K} T {T} x {x_dtype}", (1e-4 if x_dtype == 0 else 3e-5) * (K / 1536) ** 0.5)
 
 
+@pytest.mark.parametrize("T,O", [(5, 17), (5, 16 * 37 * 3), (7, 16 * 75), (5, 40)])
+def test_cluster_kernel_with_half_warps_at_different_turns(mlxq, oracle, T, O):
+    # odd tokens times odd blocks a cluster: the last rounds of the loops before the cluster's barriers, and of the block
+    # ends, are run by half a warp.  One call after the other on the same buffers, so that a CTA that left early would
+    # read the next call's sums.
+    K, gs = 12288, 64
+    fx = oracle.QuantFixture(O=O, K=K, bits=4, gs=gs, scale_type=oracle.BF16, seed=O)
+    layer = DevLayer.from_fixture(mlxq, fx)
+    x_dtype = 0 if T == 5 else 1
+    xv = oracle.RNG(T + O).floats(T * K).reshape(T, K)
+    xd = as_dtype(xv, x_dtype)
+    y = torch.full((T, O), float("nan"), device="cuda")
+    for _ in range(3):
+        layer.linear.encode(None, xd, K, y, O, T)
+    torch.cuda.synchronize()
+    mlxq.streamStatus(None, 0)
+    close(oracle, y.cpu().numpy(), fx.reference(xd.float().cpu().numpy()), f"{O}x{K} T {T}", (1e-4 if x_dtype == 0 else 3e-5) * (K / 1536) ** 0.5)
+
+
 @pytest.mark.parametrize("x_dtype,T", [(0, 9), (0, 16), (2, 16), (0, 24), (2, 24)])
 def test_batches_beyond_the_persistent_kernels_keep_fp32_products(mlxq, oracle, x_dtype, T):
     # calls that no persistent kernel holds on single CTAs, as one call or as two halves, multiply in fp32: activations of
