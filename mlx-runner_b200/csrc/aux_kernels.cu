@@ -240,10 +240,13 @@ cudaError_t launch_block_argmax(const uint32_t* pairs, int n_seg, long long T, i
 }
 
 // ---- silu_mul / gelu_tanh_mul (Kernels.swift:2004-2030): out[t, i] = act(gu[t, i]) * gu[t, cols + i] ----------------
-// `vec`: four elements per thread (rows and columns are whole 16-byte pieces), else one.
-__global__ void act_mul_kernel(const float* __restrict__ gu, long long stride, long long cols, int act, float* __restrict__ out, int vec) {
+constexpr int ACT_EACH = 4;
+// `vec`: four elements per thread as 16-byte pieces (rows and columns are whole pieces).  Else `each` elements per thread,
+// a block's width apart: one where the grid fits on the chip at once, four where it does not and the loads in flight count
+// (reads through L2 alone: 512 x 8189 with one 17.7 us, with four 8.7; 1 x 4093 1.35 / 1.64).
+__global__ void act_mul_kernel(const float* __restrict__ gu, long long stride, long long cols, int act, float* __restrict__ out, int vec, int each) {
     if (threadIdx.x == 0) dependents_may_start();
-    const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const long long i = static_cast<long long>(blockIdx.x) * (vec ? blockDim.x : each * blockDim.x) + threadIdx.x;
     const long long t = blockIdx.y;
     if (i >= (vec ? cols / 4 : cols)) return;
     wait_for_previous();
@@ -252,8 +255,17 @@ __global__ void act_mul_kernel(const float* __restrict__ gu, long long stride, l
         reinterpret_cast<float4*>(out + t * cols)[i] = make_float4(act_mul(act, g.x, u.x), act_mul(act, g.y, u.y), act_mul(act, g.z, u.z), act_mul(act, g.w, u.w));
         return;
     }
-    const float g = __ldcg(gu + t * stride + i), u = __ldcg(gu + t * stride + cols + i);
-    out[t * cols + i] = act_mul(act, g, u);
+    float g[ACT_EACH], u[ACT_EACH];
+#pragma unroll
+    for (int j = 0; j < ACT_EACH; j++) {
+        const long long k = i + static_cast<long long>(j) * blockDim.x;
+        if (j < each && k < cols) { g[j] = __ldcg(gu + t * stride + k); u[j] = __ldcg(gu + t * stride + cols + k); }
+    }
+#pragma unroll
+    for (int j = 0; j < ACT_EACH; j++) {
+        const long long k = i + static_cast<long long>(j) * blockDim.x;
+        if (j < each && k < cols) out[t * cols + k] = act_mul(act, g[j], u[j]);
+    }
 }
 
 // ---- add_rms_norm (Kernels.swift:1141-1175): h += r; y = RMSNorm(h) * w, one CTA per row.  The sum of squares is
@@ -324,8 +336,9 @@ cudaError_t launch_act_mul(const float* gu, long long stride, long long cols, lo
     if (T == 0) return cudaSuccess;
     if (T > 65535) return cudaErrorInvalidValue;
     const int vec = (cols % 4 == 0 && stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0) ? 1 : 0;
-    const long long n = vec ? cols / 4 : cols;
-    return launch_dependent(act_mul_kernel, dim3(static_cast<unsigned>((n + 255) / 256), static_cast<unsigned>(T)), dim3(256), st, gu, stride, cols, act, out, vec);
+    const int each = (cols + 255) / 256 * T > 148 * 8 ? ACT_EACH : 1;
+    const long long n = vec ? cols / 4 : (cols + each - 1) / each;
+    return launch_dependent(act_mul_kernel, dim3(static_cast<unsigned>((n + 255) / 256), static_cast<unsigned>(T)), dim3(256), st, gu, stride, cols, act, out, vec, each);
 }
 
 cudaError_t launch_add_rms_norm(float* h, const float* r, float* y, const void* w, int w_dtype, long long dim, long long rows,

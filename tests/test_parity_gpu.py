@@ -564,3 +564,16 @@ def test_dense_layers_through_the_same_handle(mlxq, oracle, wdt):
         assert torch.isnan(y[:, O]).all()
         with pytest.raises(mlxq.Unsupported):
             lin.unpackCodes(None, torch.zeros((O, K), dtype=torch.uint8, device="cuda"))
+
+
+@pytest.mark.parametrize("cols,T,pad", [(1, 1, 0), (255, 3, 1), (1021, 700, 0), (1024, 700, 3), (8189, 129, 2)])
+def test_activation_product_on_rows_that_are_no_whole_pieces(mlxq, oracle, cols, T, pad):
+    # one element per thread where the grid fits on the chip, four where it does not; ragged last blocks
+    stride = 2 * cols + pad
+    gu = oracle.RNG(cols + T).floats(T * stride).reshape(T, stride)
+    out = torch.full((T, cols), float("nan"), device="cuda")
+    mlxq.actMul(None, torch.from_numpy(gu).cuda(), stride, cols, T, mlxq.ACT_SILU, out)
+    torch.cuda.synchronize()
+    g, u = gu[:, :cols].astype(np.float64), gu[:, cols:2 * cols].astype(np.float64)
+    ref = g / (1.0 + np.exp(-g)) * u
+    assert float(np.max(np.abs(out.cpu().numpy() - ref) / np.maximum(np.abs(ref), 1e-3))) < 2e-6      # expf, a division and two products
