@@ -270,52 +270,61 @@ __global__ void act_mul_kernel(const float* __restrict__ gu, long long stride, l
 
 // ---- add_rms_norm (Kernels.swift:1141-1175): h += r; y = RMSNorm(h) * w, one CTA per row.  The sum of squares is
 // taken per thread over float4s in a strided order, then per warp, then over the warps, as the reference's threadgroup
-// does; dim is a multiple of 4 and the rows are 16-byte aligned (checked on the host).  Bound by latency -- load, reduce,
-// store -- so a row gets a thread per float4 up to 1024 threads, and a thread keeps its first NORM_KEEP float4s in
-// registers between the two passes (4096 columns: one pass over memory; 3.7 -> 2.8 us a call back to back, with the
-// dependent launch). ----------------------------------------------------------------------------------------------------
-constexpr int NORM_KEEP = 4;
-__global__ void __launch_bounds__(1024) add_rms_norm_kernel(float* __restrict__ hbuf, const float* __restrict__ r, float* __restrict__ y, const void* __restrict__ w,
-                                                            int w_dtype, int dim, long long row_stride, float eps) {
+// does; dim is a multiple of 4 and the rows are 16-byte aligned (checked on the host).  A row is summed by `nv` strands, a
+// float4 of it each up to 1024, whatever the number of rows: the order of its sums does not change with that.  Bound by
+// latency -- load, reduce, store -- while all rows are on the chip at once: a thread per strand then, which keeps its first
+// four float4s in registers between the two passes (1 x 4096: 3.7 -> 2.8 us a call back to back, with the dependent launch).
+// Beyond that, blocks of 1024 threads leave too few rows in flight and a thread takes V = 2 strands, with as many blocks on
+// an SM as keep all rows resident, or four (see launch_add_rms_norm; 512 x 4096: 9.2 us with a thread per strand, 5.8 so, 6.1
+// with 256 threads that read twice). ------------------------------------------------------------------------------------
+template <int V, int KEEP, int OCC>
+__global__ void __launch_bounds__(1024 / V, OCC) add_rms_norm_kernel(float* __restrict__ hbuf, const float* __restrict__ r, float* __restrict__ y, const void* __restrict__ w,
+                                                                int w_dtype, int dim, long long row_stride, float eps, int nv) {
     __shared__ float buf[32];
     if (threadIdx.x == 0) dependents_may_start();
     const long long row = blockIdx.x;
     float4* hr = reinterpret_cast<float4*>(hbuf + row * row_stride);
     const float4* rr = reinterpret_cast<const float4*>(r + row * row_stride);
     float4* yr = reinterpret_cast<float4*>(y + row * row_stride);
-    const int n4 = dim / 4, nt = blockDim.x;
+    const int n4 = dim / 4, nt = blockDim.x, lane = threadIdx.x & 31;
     wait_for_previous();
-    float4 kept[NORM_KEEP];
-    float ss = 0.0f;
+    float4 kept[V][KEEP];
 #pragma unroll
-    for (int k = 0; k < NORM_KEEP; k++) {
-        const int i = threadIdx.x + k * nt;
-        if (i < n4) {
+    for (int j = 0; j < V; j++)
+#pragma unroll
+        for (int k = 0; k < KEEP; k++) {
+            const int v = threadIdx.x + j * nt, i = v + k * nv;
+            if (v < nv && i < n4) {
+                const float4 a = __ldcg(hr + i), b = __ldcg(rr + i);
+                kept[j][k] = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+            }
+        }
+#pragma unroll
+    for (int j = 0; j < V; j++) {
+        const int v = threadIdx.x + j * nt;                     // (whole warps: nv is a multiple of 32)
+        if (v >= nv) break;
+        float ss = 0.0f;
+#pragma unroll
+        for (int k = 0; k < KEEP; k++) {
+            const int i = v + k * nv;
+            if (i < n4) {
+                const float4 s = kept[j][k];
+                hr[i] = s;
+                ss += s.x * s.x + s.y * s.y + s.z * s.z + s.w * s.w;
+            }
+        }
+        for (int i = v + KEEP * nv; i < n4; i += nv) {
             const float4 a = __ldcg(hr + i), b = __ldcg(rr + i);
-            kept[k] = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+            const float4 s = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+            hr[i] = s;
+            ss += s.x * s.x + s.y * s.y + s.z * s.z + s.w * s.w;
         }
-    }
 #pragma unroll
-    for (int k = 0; k < NORM_KEEP; k++) {
-        const int i = threadIdx.x + k * nt;
-        if (i < n4) {
-            const float4 v = kept[k];
-            hr[i] = v;
-            ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-        }
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) buf[v >> 5] = ss;
     }
-    for (int i = threadIdx.x + NORM_KEEP * nt; i < n4; i += nt) {
-        const float4 a = __ldcg(hr + i), b = __ldcg(rr + i);
-        const float4 v = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-        hr[i] = v;
-        ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nt >> 5;
-    if (lane == 0) buf[warp] = ss;
     __syncthreads();
-    float tot = lane < nw ? buf[lane] : 0.0f;
+    float tot = lane < nv >> 5 ? buf[lane] : 0.0f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
     const float inv = rsqrtf(tot / static_cast<float>(dim) + eps);
@@ -325,11 +334,16 @@ __global__ void __launch_bounds__(1024) add_rms_norm_kernel(float* __restrict__ 
         yr[i] = make_float4(v.x * inv * w0, v.y * inv * w1, v.z * inv * w2, v.w * inv * w3);
     };
 #pragma unroll
-    for (int k = 0; k < NORM_KEEP; k++) {
-        const int i = threadIdx.x + k * nt;
-        if (i < n4) scaled(i, kept[k]);
+    for (int j = 0; j < V; j++) {
+        const int v = threadIdx.x + j * nt;
+        if (v >= nv) break;
+#pragma unroll
+        for (int k = 0; k < KEEP; k++) {
+            const int i = v + k * nv;
+            if (i < n4) scaled(i, kept[j][k]);
+        }
+        for (int i = v + KEEP * nv; i < n4; i += nv) scaled(i, hr[i]);
     }
-    for (int i = threadIdx.x + NORM_KEEP * nt; i < n4; i += nt) scaled(i, hr[i]);
 }
 
 cudaError_t launch_act_mul(const float* gu, long long stride, long long cols, long long T, int act, float* out, cudaStream_t st) {
@@ -345,8 +359,15 @@ cudaError_t launch_add_rms_norm(float* h, const float* r, float* y, const void* 
                                 long long row_stride, float eps, cudaStream_t st) {
     if (rows == 0) return cudaSuccess;
     const long long n4 = dim / 4;
-    const unsigned threads = static_cast<unsigned>(n4 < 1024 ? (n4 + 31) / 32 * 32 : 1024);
-    return launch_dependent(add_rms_norm_kernel, dim3(static_cast<unsigned>(rows)), dim3(threads), st, h, r, y, w, w_dtype, static_cast<int>(dim), row_stride, eps);
+    const int nv = static_cast<int>(n4 < 1024 ? (n4 + 31) / 32 * 32 : 1024);
+    // In strands: what a thread per strand holds with one block of 1024 on an SM (two where a row is several turns of every
+    // thread: 200 x 16384 10.2 us against 11.9), then what three blocks of half the threads hold (300 x 4096: 4.9 us; with
+    // room for four 5.5, since the registers do not hold the row).
+    const long long strands = rows * nv, wave = 148 * 1024;
+    const int V = strands <= (n4 >= 2048 ? 2 : 1) * wave ? 1 : 2;
+    const auto kernel = V == 1 ? add_rms_norm_kernel<1, 4, 1> : strands <= 3 * wave ? add_rms_norm_kernel<2, 1, 3> : add_rms_norm_kernel<2, 1, 4>;
+    const unsigned threads = static_cast<unsigned>((nv / V + 31) / 32 * 32);
+    return launch_dependent(kernel, dim3(static_cast<unsigned>(rows)), dim3(threads), st, h, r, y, w, w_dtype, static_cast<int>(dim), row_stride, eps, nv);
 }
 
 }  // namespace mlxq

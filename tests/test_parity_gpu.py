@@ -577,3 +577,26 @@ def test_activation_product_on_rows_that_are_no_whole_pieces(mlxq, oracle, cols,
     g, u = gu[:, :cols].astype(np.float64), gu[:, cols:2 * cols].astype(np.float64)
     ref = g / (1.0 + np.exp(-g)) * u
     assert float(np.max(np.abs(out.cpu().numpy() - ref) / np.maximum(np.abs(ref), 1e-3))) < 2e-6      # expf, a division and two products
+
+
+@pytest.mark.parametrize("dim", [4, 132, 2048, 4096, 8196, 20480])
+def test_add_rms_norm_of_a_row_does_not_depend_on_the_rows_beside_it(mlxq, oracle, dim):
+    # many rows take other launch shapes than few: the bits of a row stay the same, and are the oracle's to the rounding of
+    # the sum of squares (strands of dim / 1024 terms, then ten pairwise steps: 2^-24 * 20)
+    rows = 700
+    rng = oracle.RNG(dim)
+    h, r, w = (rng.floats(n * dim).reshape(n, dim) for n in (rows, rows, 1))
+    stride, outs = dim + 4, []
+    for part in (1, 200, rows):
+        hd, rd = (torch.full((part, stride), float("nan"), device="cuda") for _ in range(2))
+        hd[:, :dim], rd[:, :dim] = torch.from_numpy(h[:part]).cuda(), torch.from_numpy(r[:part]).cuda()
+        yd = torch.zeros((part, stride), device="cuda")
+        mlxq.addRMSNorm(None, hd, rd, yd, torch.from_numpy(w[0]).cuda(), dim, part, stride, 1e-5)
+        torch.cuda.synchronize()
+        outs.append((hd[:, :dim].cpu().numpy(), yd[:, :dim].cpu().numpy()))
+    for hd, yd in outs[:2]:
+        assert np.array_equal(hd, outs[2][0][:len(hd)]) and np.array_equal(yd, outs[2][1][:len(yd)])
+    href = h + r
+    assert np.array_equal(outs[2][0], href)
+    ref = href / np.sqrt((href.astype(np.float64) ** 2).mean(axis=1, keepdims=True) + 1e-5) * w
+    assert float(np.max(np.abs(outs[2][1] - ref) / np.maximum(np.abs(ref), 1e-3))) < 20 * 2.0 ** -24
