@@ -56,7 +56,7 @@ dense_mv_kernel(const void* __restrict__ w, int w_dtype, const void* __restrict_
         for (int t = 0; t < NT; t++) acc[r][t] = 0.0f;
     }
     const int K8 = K & ~7;
-#pragma unroll(NT <= 2 && ROWS == 1 ? 4 : 2)
+#pragma unroll 1
     for (int k = lane * 8; k < K8; k += 256) {
         float wv[ROWS][8];
 #pragma unroll
@@ -102,14 +102,13 @@ void launch_tokens(int nt, unsigned grid, cudaStream_t st, const void* w, int w_
     dense_mv_kernel<NT, ROWS><<<grid, DENSE_WARPS * 32, 0, st>>>(w, w_dtype, bias, bias_dtype, x, x_dtype, x_stride, y, y_dtype, y_stride, O, K, w_vec, x_vec);
 }
 
-// Rows per warp.  More of them save activation reads but leave fewer warps, which few rows or few tokens do not pay for
-// (1 / 2 / 4 rows per warp: 32000 x 4096 with 4 tokens 167 / 139 / 195 us, with 8 351 / 305 / 269; 4096 x 4096 with 2 tokens
-// 19 / 27 / 42, with 8 74 / 50 / 70; 2048 x 2048 with 8 tokens 21 / 24 / 32).
-int rows_per_warp(int tokens, int O) {
-    if (tokens >= 5) return O >= 24576 ? 4 : O >= 4096 ? 2 : 1;
-    if (tokens >= 2) return O >= (tokens == 2 ? 24576 : 8192) ? 2 : 1;
-    return 1;
-}
+// Rows per warp.  Two save activation reads but leave half as many warps, which few rows or few tokens do not pay for.
+// Times over those of a row per warp with the tokens not compiled in (bf16 weights, 512 ... 8192 columns, geometric mean):
+//   fp32 tokens, 1 / 2 rows per warp:  2 tokens  4096 rows 0.90 / 1.03, 32000 0.83 / 0.85;  8 tokens  0.98 / 0.98, 0.94 / 0.75
+//   bf16 tokens:                       2 tokens  4096 rows 0.86 / 1.09, 32000 0.72 / 0.88;  8 tokens  0.91 / 1.05, 0.86 / 0.83
+// and from 6144 rows on two win from 3 fp32 or 4 bf16 tokens on (3 bf16 tokens 0.64 ... 0.84 / 0.72 ... 0.91).  Four rows per
+// warp, and two turns of the loop in flight, cost registers and with them warps: 8 bf16 tokens with either 1.06 ... 1.35.
+int rows_per_warp(int tokens, int O) { return tokens >= 3 && O >= 6144 ? 2 : 1; }
 
 }  // namespace
 
@@ -122,7 +121,7 @@ cudaError_t launch_dense(const void* w, int w_dtype, const void* bias, int bias_
         const int tt = static_cast<int>(T - t0 < DENSE_TOKENS ? T - t0 : DENSE_TOKENS);
         const int rows = rows_per_warp(tt, O);
         const unsigned grid = static_cast<unsigned>((O + DENSE_WARPS * rows - 1) / (DENSE_WARPS * rows));
-        const auto launch = rows == 4 ? launch_tokens<DENSE_TOKENS, 4> : rows == 2 ? launch_tokens<DENSE_TOKENS, 2> : launch_tokens<DENSE_TOKENS, 1>;
+        const auto launch = rows == 2 ? launch_tokens<DENSE_TOKENS, 2> : launch_tokens<DENSE_TOKENS, 1>;
         launch(tt, grid, st, w, w_dtype, bias, bias_dtype, static_cast<const char*>(x) + static_cast<size_t>(t0) * x_stride * xsz, x_dtype, x_stride,
                static_cast<char*>(y) + static_cast<size_t>(t0) * y_stride * dtype_size(y_dtype), y_dtype, y_stride, O, K, w_vec, x_vec);
         const cudaError_t e = cudaGetLastError();

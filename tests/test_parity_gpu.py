@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import DevLayer, as_dtype, dev, run
+from helpers import TORCH_DT, DevLayer, as_dtype, dev, run
 
 synth = importlib.import_module("mlx-runner_b200.synth")
 
@@ -600,3 +600,24 @@ def test_add_rms_norm_of_a_row_does_not_depend_on_the_rows_beside_it(mlxq, oracl
     assert np.array_equal(outs[2][0], href)
     ref = href / np.sqrt((href.astype(np.float64) ** 2).mean(axis=1, keepdims=True) + 1e-5) * w
     assert float(np.max(np.abs(outs[2][1] - ref) / np.maximum(np.abs(ref), 1e-3))) < 20 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("O,T,x_dtype", [(6143, 3, 0), (6145, 3, 2), (6151, 8, 0), (6145, 11, 1), (4097, 8, 2), (33, 2, 0)])
+@pytest.mark.parametrize("w_dtype", [0, 1, 2])
+def test_dense_rows_per_warp_at_their_edges(mlxq, oracle, O, T, x_dtype, w_dtype):
+    # one and two rows per warp on either side of their bound, odd row counts (the last warp's second row is past the end), a
+    # second turn of fewer tokens, a row bias, padded outputs, a ragged last chunk of K
+    K, stride = 516 if T == 3 else 520, 536                        # (rows of whole 16-byte pieces and not)
+    rng = oracle.RNG(O + T)
+    w = as_dtype(rng.floats(O * K).reshape(O, K), w_dtype)
+    bias = as_dtype(rng.floats(O), w_dtype)
+    x = torch.zeros((T, stride), dtype=TORCH_DT[x_dtype], device="cuda")
+    x[:, :K] = as_dtype(rng.floats(T * K).reshape(T, K), x_dtype)
+    lin = mlxq.Linear(w, None, None, bias, inDim=K)
+    y = torch.full((T, O + 3), float("nan"), device="cuda")
+    lin.encode(None, x, stride, y, O + 3, T)
+    torch.cuda.synchronize()
+    ref = x[:, :K].double() @ w.double().t() + bias.double()
+    # fp32 sums of 520 terms in 32 lanes: 17 roundings each and five more, 2^-24 * 22 of the terms' magnitude (below 2 * |y| + 4)
+    assert float(((y[:, :O].double() - ref).abs() / (ref.abs() + 4.0)).max()) < 22 * 2.0 ** -23
+    assert torch.isnan(y[:, O:]).all()
