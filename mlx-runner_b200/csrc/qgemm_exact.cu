@@ -662,14 +662,17 @@ int segments(int m_tiles, int k_stages, int least) {
     return best;
 }
 
-// 8-bit rows of more than 8192 codes with 16-bit activations, which the CUDA-core kernel serves otherwise: segments of 24
-// drain steps at most, 16 of them at most, so that the error is not above that kernel's.  The products are exact here and
-// the roundings of the running sum are what is left; in sums of 48 and 96 steps they came to 1.34e-7 and 1.82e-7 of the
-// result (12288 codes in groups of 64 and 32), in sums of 24 to 1.1e-7 and 1.2e-7, there to 1.2e-7.  (4096 x 12288 with 384
-// bf16 tokens: 129 -> 141 us in groups of 64, 209 -> 260 in groups of 32.)
+// With 16-bit activations the products are exact and the roundings of the running sum are what is left; they grow with its
+// length, and the kernels that serve such calls otherwise have shorter sums.  So that the error is not above theirs:
+// * 8-bit rows of more than 8192 codes, the CUDA-core kernel's: segments of 24 drain steps at most, 16 of them at most.  In
+//   sums of 48 and 96 steps the error was 1.34e-7 and 1.82e-7 of the result (12288 codes in groups of 64 and 32), in sums of
+//   24 it is 1.1e-7 and 1.2e-7, there 1.2e-7.  (4096 x 12288 with 384 bf16 tokens: 125 -> 150 us in groups of 64, 206 -> 252
+//   in groups of 32.)
+// * 6 and 8 bits in groups of 32: 64 steps.  (14336 x 4096 in sums of 128 2.1e-7, of 64 1.5e-7; the token-major kernel 1.7e-7.)
 int least_segments(const GemmLayer& L, int parts) {
-    if (L.bits != 8 || parts != 1 || L.K <= 8192) return 1;
-    const int steps = L.K / (L.gs == 32 ? 32 : BK), s = (steps + 23) / 24;
+    if (L.bits < 6 || parts != 1) return 1;
+    const int steps = L.K / (L.gs == 32 ? 32 : BK), limit = L.bits == 8 && L.K > 8192 ? 24 : L.gs == 32 ? 64 : steps;
+    const int s = (steps + limit - 1) / limit;
     return s < 16 ? s : 16;
 }
 
