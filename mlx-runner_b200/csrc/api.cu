@@ -324,13 +324,18 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
         };
         const int64_t h0 = T / 2;
         const int fit = persistent && !rsmem && T >= 4 ? fits_persistent(h0) * fits_persistent(T - h0) : 0;
-        if (persistent && !rsmem && T >= 2 && !(mode && strcmp(mode, "pipe") == 0) && (fit == 4 || peer || (x_up && !fit))) {
-            // Too many staged activation columns for a CTA's shared memory (long rows): the token-major kernel with K split
-            // over a cluster, in the place of two of its calls with half the tokens.  Not in the place of another kernel: the
-            // one-token kernel's sums are the more exact ones (8 bits, 4096 x 12288, 3 fp32 tokens: 2.0e-7 of the result
-            // against 5.5e-7), and the CUDA-core kernel multiplies in fp32, at any magnitude of the activations.
+        // Too many staged activation columns for a CTA's shared memory (long rows): the token-major kernel with K split over a
+        // cluster, in the place of two of its calls with half the tokens.  Not in the place of the one-token kernel, whose sums
+        // are the more exact ones (8 bits, 4096 x 12288, 3 fp32 tokens: 2.0e-7 of the result against 5.5e-7).  Where no
+        // persistent kernel would do, the others take activations of any magnitude: there the cluster scales them, and serves
+        // what its error is no larger for than theirs (mean over shapes and batches of its error over theirs: 2 to 6 bits
+        // 0.59 ... 0.95, 8 bits 1.00 with fp32 activations and 1.50 with 16-bit ones; over the register-fed kernel's, which
+        // fits some three-token calls, 1.15 at 6 bits).  4096 x 14336, 3 fp32 tokens, 4 bits: 240 -> 24 us.
+        const int bits = parts[0]->bits;
+        const bool as_exact = bits <= 5 || (bits == 6 && !smem) || (bits == 8 && mp.split == 2);
+        if (persistent && !rsmem && T >= 2 && !(mode && strcmp(mode, "pipe") == 0) && (fit == 4 || peer || (!fit && (as_exact || x_up)))) {
             TokPlan tp;
-            const size_t tsmem = qmv_tok_plan(parts[0]->bits, mp, static_cast<int>(T), device_sm_count(parts[0]->device), tp, true);
+            const size_t tsmem = qmv_tok_plan(bits, mp, static_cast<int>(T), device_sm_count(parts[0]->device), tp, fit == 4 ? 1 : 2);
             if (tsmem) {
                 const cudaError_t err = launch_qmv_tok(parts[0]->bits, mp, tp, tsmem, parts[0]->device, st);
                 if (err != cudaSuccess) return cuda_fail(err, "qmv (token-major, cluster) launch");

@@ -85,6 +85,14 @@ template <> struct XLoad<__nv_bfloat16> {
     }
 };
 
+// A token's power of two (biased exponent; the inverse's is 254 - it, never that of a subnormal number), from its largest
+// magnitude: that comes to [2^14, 2^15), so that no activation overflows fp16 and the low fp16 part of an fp32 one is no
+// subnormal number wherever that matters (what is lost lies below 2^-40 of the largest).  One for a row with an infinity.
+__device__ __forceinline__ uint32_t token_scale_exponent(float largest) {
+    const uint32_t e = __float_as_uint(largest) >> 23;                        // (sign bit clear)
+    return e == 255u ? 127u : min(268u - e, 253u);
+}
+
 // ---- generic decoder: eight codes from BITS bytes at any byte address --------------------------------
 // Code i of the chunk is bits [i*BITS, (i+1)*BITS) of the little-endian value of those bytes.
 template <int BITS>

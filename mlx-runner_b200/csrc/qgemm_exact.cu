@@ -474,15 +474,8 @@ struct ExactStage {
     unsigned x_blocks;
 };
 
-// A token's power of two: its largest magnitude comes to [2^14, 2^15), so that no activation overflows fp16 and the low
-// parts are no subnormal numbers wherever that matters (what is lost lies below 2^-40 of the largest).  Unscaled, an
-// activation of 1e5 became infinity, and fp32 ones of 1e-4 kept 13 of their 24 bits.  fp16 activations are what they
-// are: factor one, as for a row with an infinity.
-__device__ __forceinline__ uint32_t scale_exponent(float largest) {
-    const uint32_t e = __float_as_uint(largest) >> 23;                        // (sign bit clear)
-    return e == 255u ? 127u : min(268u - e, 253u);                            // biased; the inverse is 254 - it, never subnormal
-}
-
+// Activations are scaled by a power of two per token (token_scale_exponent): unscaled, one of 1e5 became infinity, and fp32
+// ones of 1e-4 kept 13 of their 24 bits.  fp16 activations are what they are: factor one.
 constexpr int STAGE_THREADS = 256;
 constexpr int STAGE_KEEP = 6;                // chunks of a thread that stay in registers between the two passes: 12288 codes
 
@@ -524,7 +517,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) exact_stage_kernel(const ExactS
                 __syncthreads();
 #pragma unroll
                 for (int w = 0; w < STAGE_THREADS / 32; w++) largest = fmaxf(largest, warp_max[w]);
-                const uint32_t e = scale_exponent(largest);
+                const uint32_t e = token_scale_exponent(largest);
                 factor = __uint_as_float(e << 23);
                 inverse = __uint_as_float((254u - e) << 23);
             }

@@ -21,7 +21,7 @@ bool supported(int bits, int gs) {
     return nm >= 2 && nm % 2 == 0;
 }
 
-template <int BITS, int GS, int NP, int DEPTH_CT, bool CLUSTER>
+template <int BITS, int GS, int NP, int DEPTH_CT, bool CLUSTER, bool SCALED = false>
 cudaError_t launch_one(const MmaParams& p, const TokPlan& tp, size_t smem, int device, cudaStream_t st) {
     if constexpr (!TokUnit<BITS, GS>::SUPPORTED) {
         return cudaErrorNotSupported;
@@ -33,7 +33,7 @@ cudaError_t launch_one(const MmaParams& p, const TokPlan& tp, size_t smem, int d
         {
             std::lock_guard<std::mutex> lk(mu);
             if (!done[device]) {
-                const cudaError_t e = cudaFuncSetAttribute(qmv_tok_kernel<BITS, GS, NP, DEPTH_CT, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_WHOLE);
+                const cudaError_t e = cudaFuncSetAttribute(qmv_tok_kernel<BITS, GS, NP, DEPTH_CT, CLUSTER, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_WHOLE);
                 if (e != cudaSuccess) return e;
                 done[device] = true;
             }
@@ -55,7 +55,7 @@ cudaError_t launch_one(const MmaParams& p, const TokPlan& tp, size_t smem, int d
         }
         cfg.attrs = la;
         cfg.numAttrs = static_cast<unsigned>(n);
-        return cudaLaunchKernelEx(&cfg, qmv_tok_kernel<BITS, GS, NP, DEPTH_CT, CLUSTER>, p, tp);
+        return cudaLaunchKernelEx(&cfg, qmv_tok_kernel<BITS, GS, NP, DEPTH_CT, CLUSTER, SCALED>, p, tp);
     }
 }
 
@@ -63,6 +63,7 @@ template <int BITS, int GS, int NP>
 cudaError_t launch_depth(const MmaParams& p, const TokPlan& tp, size_t smem, int device, cudaStream_t st) {
     // the width's usual ring depth is compiled in; a shallower ring (shared memory short) takes the general instance
     constexpr int usual = GS * BITS / 32 >= 16 ? 4 : 8;
+    if (tp.scaled) return launch_one<BITS, GS, NP, 0, true, true>(p, tp, smem, device, st);
     if (tp.kz > 1 || !planned_width<BITS>()) return tp.depth == usual ? launch_one<BITS, GS, NP, usual, true>(p, tp, smem, device, st) : launch_one<BITS, GS, NP, 0, true>(p, tp, smem, device, st);
     if constexpr (planned_width<BITS>())
         return tp.depth == usual ? launch_one<BITS, GS, NP, usual, false>(p, tp, smem, device, st) : launch_one<BITS, GS, NP, 0, false>(p, tp, smem, device, st);
@@ -94,7 +95,7 @@ int cluster_capacity(int kz, int sms) {
     const int slot = kz == 2 ? 0 : kz == 4 ? 1 : 2;
     std::lock_guard<std::mutex> lk(mu);
     if (!cached[dev][slot]) {
-        const auto kernel = qmv_tok_kernel<4, 64, 1, 4, true>;
+        const auto kernel = qmv_tok_kernel<4, 64, 1, 4, true, false>;
         int n = 0;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(sms / kz * kz));
@@ -123,7 +124,7 @@ int k_split(int n_blocks) { return n_blocks <= 1024 ? 4 : 2; }
 
 }  // namespace
 
-size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& tp, bool clusters) {
+size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& tp, int clusters) {
     const QmvParams& q = p.q;
     if (tokens < 1 || q.total_rows < 1 || p.xn < 1 || p.xn > 16) return 0;
     if (q.gs != 32 && q.gs != 64 && q.gs != 128) return 0;
@@ -144,6 +145,7 @@ size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& 
     const int warps = TOK_WARPS;
     tp.n_blocks = (q.total_rows + 15) / 16;
     tp.tp = tokens + 1;
+    tp.scaled = clusters == 2;
     long long best_cost = -1;
     size_t best_total = 0;
     // (a split whose slices still do not fit a CTA's shared memory is doubled)
@@ -166,12 +168,13 @@ size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& 
         tp.off_zero = off; off += PIPE_ZERO_BYTES;
         const int cta_blocks = (tp.n_blocks + n_cl - 1) / n_cl;
         tp.off_z = off; if (kz > 1) off += cta_blocks * tokens * 64;
+        tp.off_scale = off; if (kz > 1) off += 3 * 64;
         tp.off_part = off;
         const int off_fixed = off;
         // K split and ring depth: the split that leaves the longest-working warp the least to do, among those whose
         // slices are equal, even, and at least two groups long; the deepest ring that fits.
         for (int parities = 2; parities >= 1 && best_cost < 0; parities--)
-        for (int ks = 1; ks <= warps; ks *= 2) {
+        for (int ks = tp.scaled ? 4 : 1; ks <= warps; ks *= 2) {
             const int off_tab = align_up(off_fixed + parities * warps * 16 * tp.tp * 4, 128);
             // slices are cut at even groups; the shortest must hold a pair, the longest sets the tables' size
             int slice = 0, slice_min = groups;

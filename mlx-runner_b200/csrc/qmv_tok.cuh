@@ -32,6 +32,9 @@ constexpr int TOK_WARPS = 16;
 struct TokPlan {
     int kz, kz_shift;    // CTAs (a cluster) that share a block along K and its log2
     int off_z;           // kz > 1: the CTA's sums [block of the cluster][token][16 rows] floats
+    int scaled;          // kz > 1: activations are scaled by a power of two per token, which the outputs undo (K is split over four
+                         // warps at least then: short sums, as the call stands in for kernels that have them)
+    int off_scale;       // ... the tokens' largest magnitudes (bits), their factors, the inverses: three times sixteen words
     int ks, ks_shift;    // warps that share a block along the CTA's slice of K and its log2
     int depth;           // ring slots (groups in flight) per warp: 8, 4 or 2
     int ntab;            // buffers of the per-block (scale, bias) cells: blocks the copy cursor may run ahead, plus two
@@ -100,8 +103,9 @@ __device__ __forceinline__ float cluster_load(uint32_t addr, int rank) {
 // DEPTH_CT: the ring depth when it is the width's usual one (compiled in), 0 when the planner had to take a shallower ring.
 // CLUSTER: K may be split over the CTAs of a cluster.  Compiled out for single CTAs at the widths whose codes straddle bytes,
 // where the extra code cost 0.8 %; at the others the one instance serves both and is the faster one (step of 36 4-bit
-// layers, 6 tokens: 3343 us against 3407 with an instance for each).
-template <int BITS, int GS, int NP, int DEPTH_CT, bool CLUSTER>
+// layers, 6 tokens: 3343 us against 3407 with an instance for each).  SCALED: the cluster's instance for activations of any
+// magnitude (scaled by a power of two per token), which cost the others 1 to 2 % where it was compiled into them.
+template <int BITS, int GS, int NP, int DEPTH_CT, bool CLUSTER, bool SCALED>
 __global__ void __launch_bounds__(TOK_WARPS * 32, 1)
 qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokPlan tp) {
     using U = TokUnit<BITS, GS>;
@@ -263,7 +267,45 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
         const int cpr = cg << (GSH - 3), total_chunks = T * cpr, k0 = gb << GSH;
         constexpr int cpg = GS / 8;
         constexpr int SU = 4;                                  // chunks whose loads are in flight together
-        const bool f16_fast = (BITS == 4 || BITS == 8) && split == 1 && q.x_dtype == DT_F16;
+        const bool f16_fast = (BITS == 4 || BITS == 8) && split == 1 && q.x_dtype == DT_F16 && !SCALED;
+        if constexpr (SCALED) {
+            // every token's largest magnitude: this CTA's slice, then the cluster's
+            unsigned* top = reinterpret_cast<unsigned*>(smem_tok + tp.off_scale);
+            if (threadIdx.x < 16) top[threadIdx.x] = 0u;
+            __syncthreads();
+            for (int base = 0; base < total_chunks; base += NT) {
+                const int idx = base + threadIdx.x, tok = tp.cpr_shift >= 0 ? idx >> tp.cpr_shift : idx / cpr, k = (idx - tok * cpr) * 8;
+                float m = 0.0f;
+                if (idx < total_chunks) {
+                    float v[8];
+                    load8_coherent(q.x, q.x_dtype, static_cast<size_t>(tok) * q.x_stride + k0 + k, v);
+                    if (q.x_up != nullptr) {
+                        float up[8];
+                        load8_coherent(q.x_up, DT_F32, static_cast<size_t>(tok) * q.x_stride + k0 + k, up);
+#pragma unroll
+                        for (int i = 0; i < 8; i++) v[i] = act_mul(q.x_act, v[i], up[i]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; i++) m = fmaxf(m, fabsf(v[i]));
+                }
+                if (__all_sync(0xffffffffu, tok == __shfl_sync(0xffffffffu, tok, 0))) {
+                    const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+                    if (lane == 0 && idx < total_chunks) atomicMax(top + tok, wm);
+                } else if (idx < total_chunks) {
+                    atomicMax(top + tok, __float_as_uint(m));
+                }
+            }
+            __syncthreads();
+            cluster_barrier();
+            if (threadIdx.x < static_cast<unsigned>(T)) {
+                float m = 0.0f;
+                for (int rk = 0; rk < kz; rk++) m = fmaxf(m, cluster_load(smem_u32(top + threadIdx.x), rk));
+                const uint32_t e = token_scale_exponent(m);
+                reinterpret_cast<float*>(top)[16 + threadIdx.x] = __uint_as_float(e << 23);
+                reinterpret_cast<float*>(top)[32 + threadIdx.x] = __uint_as_float((254u - e) << 23);
+            }
+            __syncthreads();
+        }
         for (int base = 0; base < total_chunks; base += NT * SU) {
             uint4 ra[SU], rb[SU];
 #pragma unroll
@@ -299,6 +341,11 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
                         load8_coherent(q.x_up, DT_F32, static_cast<size_t>(tok) * q.x_stride + k0 + k, up);
 #pragma unroll
                         for (int i = 0; i < 8; i++) v[i] = act_mul(q.x_act, v[i], up[i]);
+                    }
+                    if constexpr (SCALED) {
+                        const float f = reinterpret_cast<const float*>(smem_tok + tp.off_scale)[16 + tok];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) v[i] *= f;
                     }
 #pragma unroll
                     for (int i = 0; i < 8; i++) sum += v[i];
@@ -396,6 +443,14 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
                 uint32_t s0, s1, b0, b1;
                 asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(s0), "=r"(s1), "=r"(b0), "=r"(b1) : "r"(cell));
                 cell += 512;
+                if constexpr (SCALED || (CLUSTER && planned_width<BITS>())) {
+                    // the previous window's bias term joins the running sum, so that that holds little more than the result's
+                    // share: the two terms are each some times larger, and every rounding is in proportion to what is held
+#pragma unroll
+                    for (int ps = 0; ps < NP; ps++)
+#pragma unroll
+                        for (int i = 0; i < 4; i++) { yacc[ps][i] = fmaf(yb[ps][i], 1.0f / 16777216.0f, yacc[ps][i]); yb[ps][i] = 0.0f; }
+                }
                 // bias term of the window's eight groups: k slot t is group 2t, slot t + 4 is group 2t + 1
                 uint32_t a0, a1, a2, a3;
                 if (s_f16) {
@@ -546,6 +601,7 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
             float v = 0.0f;
             for (int rk = 0; rk < kz; rk++) v += cluster_load(z + idx * 4, rk);
             const int bt = idx >> 4, blk = bt / T;
+            if constexpr (SCALED) v *= reinterpret_cast<const float*>(smem_tok + tp.off_scale)[32 + bt - blk * T];
             finish((cid + blk * n_cl) * 16 + (idx & 15), bt - blk * T, v);
         }
         cluster_barrier();                                      // nobody leaves while its sums are being read
@@ -555,8 +611,8 @@ qmv_tok_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TokP
 }
 
 // Plans a call of the token-major kernel; returns the shared memory it needs, 0 when the call is not one it serves.
-// `clusters`: a plan with K split over the CTAs of a cluster, or else one for single CTAs.
-size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& tp, bool clusters = false);
+// `clusters`: 0 a plan for single CTAs, 1 one with K split over the CTAs of a cluster, 2 that with scaled activations.
+size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& tp, int clusters = 0);
 cudaError_t launch_qmv_tok(int bits, const MmaParams& p, const TokPlan& tp, size_t smem, int device, cudaStream_t st);
 
 }  // namespace mlxq

@@ -214,6 +214,44 @@ def test_cluster_kernel_with_half_warps_at_different_turns(mlxq, oracle, T, O):
     close(oracle, y.cpu().numpy(), fx.reference(xd.float().cpu().numpy()), f"{O}x{K} T {T}", (1e-4 if x_dtype == 0 else 3e-5) * (K / 1536) ** 0.5)
 
 
+@pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
+@pytest.mark.parametrize("x_dtype,T", [(0, 7), (0, 8), (1, 12), (2, 13)])
+def test_cluster_kernel_at_any_magnitude(mlxq, oracle, bits, x_dtype, T):
+    # batches that the clusters serve in the place of kernels that multiply in fp32: tokens of 1e-30 ... 1e30 side by side, one
+    # of zeros, one whose elements span ten orders of magnitude; in fp16 down to its subnormal numbers.  A token's power of two
+    # leaves what lies above 2^-40 of its largest element as exact as at magnitude one; the bar there is that of the sums: the
+    # uncentred codes' are up to four times the result's at 2 bits, 14336 terms in 16 slices, 2^-24 * sqrt(14336 / 16 / 8) * 4
+    # and the bias term's as much again: 5e-6.
+    if bits == 8 and x_dtype != 0:
+        T = 8                                                      # (8 bits, 16-bit activations: two half batches, no cluster beyond)
+    K, gs = 14336, 64
+    for O in (40, 16 * 37 + 1):
+        fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=gs, scale_type=oracle.BF16, seed=bits + O)
+        layer = DevLayer.from_fixture(mlxq, fx)
+        x = oracle.RNG(T + bits).floats(T * K).reshape(T, K)
+        mags = [1.0] * 3 if bits == 8 and x_dtype != 0 else [1e-6, 1e-3, 3e4] if x_dtype == 1 else [1e-30, 1e-5, 1e30]
+        for t, m in enumerate(mags):
+            x[t] = x[t] * np.float32(m)
+        x[3] = 0.0
+        if x_dtype != 1 and bits != 8:
+            x[4] = x[4] * np.exp(np.linspace(0.0, 23.0, K)).astype(np.float32)
+        xd = as_dtype(x, x_dtype)
+        y = torch.full((T, O + 3), float("nan"), device="cuda")
+        layer.linear.encode(None, xd, K, y, O + 3, T)
+        torch.cuda.synchronize()
+        mlxq.streamStatus(None, 0)
+        got = y.cpu().numpy()[:, :O].astype(np.float64)
+        w = np.repeat(oracle.to_float(fx.scales_raw, oracle.BF16), gs, axis=1).astype(np.float64) * fx.q + \
+            np.repeat(oracle.to_float(fx.biases_raw, oracle.BF16), gs, axis=1).astype(np.float64)
+        ref = xd.double().cpu().numpy() @ w.T
+        for t in range(T):
+            if t == 3:
+                assert not got[t].any()
+                continue
+            err = float(np.linalg.norm(got[t] - ref[t]) / np.linalg.norm(ref[t]))
+            assert err < 5e-6, f"bits {bits} x dtype {x_dtype} {O}x{K} token {t} of {T}: {err}"
+
+
 @pytest.mark.parametrize("x_dtype,T", [(0, 9), (0, 16), (2, 16), (0, 24), (2, 24)])
 def test_batches_beyond_the_persistent_kernels_keep_fp32_products(mlxq, oracle, x_dtype, T):
     # calls that no persistent kernel holds on single CTAs, as one call or as two halves, multiply in fp32: activations of
