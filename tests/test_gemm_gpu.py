@@ -9,8 +9,8 @@ that weight rounding plus the fp32 accumulation order.  Bars:
   ||got-ref|| / ||ref|| < 1e-3;
 * the reference fixture's much larger magnitudes (|w| ~ 0.3, |y| ~ 5-20): normwise < 5e-4 (= 2 * 2^-12);
   the element-wise metric, which divides the absolute error by max(1,|ref|) even where |ref| is small
-  next to the row's terms, must stay < 1.5e-2.  (fp32 activations never take this path: they use the
-  fp32 CUDA-core kernel and meet 1e-3 element-wise, tests/test_parity_gpu.py.)"""
+  next to the row's terms, must stay < 1.5e-2.  (fp32 activations never take this path: they, and all
+  other widths, take the full-precision GEMM, whose bars stand with its tests.)"""
 import importlib
 
 import numpy as np
@@ -199,7 +199,7 @@ def test_prepared_table_changes_nothing(mlxq, oracle):
 @pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
 def test_full_precision_gemm_at_its_edges(mlxq, oracle, bits):
     # the GEMM behind batches whose operands may not be rounded to fp16: one step of K and more, all group sizes, one to
-    # several row tiles and tokens tiles of 32 / 64 / 128, K split over CTAs (K = 2048: eight segments) and not, a row
+    # several row tiles and tokens tiles of 32 / 64 / 128, K split over CTAs (K = 2048: four segments) and not, a row
     # bias, strided rows with NaN padding.  The bound: an activation is kept to 2^-22 (two fp16 numbers), each of up to eight
     # tensor-core steps of a group drops what lies below 2^-25 of its sum, the rest is fp32: 2^-22 + 8 * 2^-25 < 5e-7 of
     # the terms, which cancel by less than two -- 1e-6 normwise.
@@ -365,3 +365,78 @@ def test_ordinary_launches_give_the_same_bits(mlxq, tmp_path):
         got.append(torch.load(out))
     for key, (y, a) in got[0].items():
         assert torch.equal(y, got[1][key][0]) and torch.equal(a, got[1][key][1]), key
+
+
+def _sampled(oracle, fx, xr, rows, tokens):
+    """The oracle's outputs of some rows for some tokens."""
+    return oracle.qmatmul(fx.packed[rows], fx.scales_raw[rows], fx.biases_raw[rows], oracle.BF16, np.ascontiguousarray(xr[tokens]), fx.K, fx.bits, fx.gs)
+
+
+@pytest.mark.parametrize("bits", [2, 5, 8])
+def test_full_precision_gemm_in_eight_segments(mlxq, oracle, bits):
+    # 4096 codes on three row tiles: K over eight CTAs
+    O, K, T = 300, 4096, 70
+    fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=64, scale_type=oracle.BF16, seed=bits)
+    layer = DevLayer.from_fixture(mlxq, fx)
+    for x_dtype in (0, 2):
+        x = oracle.RNG(T).floats(T * K).reshape(T, K)
+        xr = as_dtype(x, x_dtype).float().cpu().numpy()
+        got = run(layer, x, T, x_dtype=x_dtype, y_stride=O + 3)
+        ref = _ref(oracle, fx, xr, K, bits, 64, oracle.BF16)
+        assert float(np.linalg.norm(got - ref) / np.linalg.norm(ref)) < 1e-6
+    mlxq.streamStatus(None, 0)
+
+
+@pytest.mark.parametrize("K", [128, 256, 384])
+def test_full_precision_gemm_on_short_4_bit_rows(mlxq, oracle, K):
+    # 4-bit layers with 16-bit activations take it below 512 codes (one fp16 part, codes in the permuted order)
+    O, T = 264, 90
+    fx = oracle.QuantFixture(O=O, K=K, bits=4, gs=64, scale_type=oracle.BF16, with_bias=True, seed=K)
+    layer = DevLayer.from_fixture(mlxq, fx)
+    for x_dtype in (1, 2):
+        x = oracle.RNG(T + K).floats(T * K).reshape(T, K)
+        xr = as_dtype(x, x_dtype).float().cpu().numpy()
+        got = run(layer, x, T, x_dtype=x_dtype, x_stride=K + 8)
+        ref = _ref(oracle, fx, xr, K, 4, 64, oracle.BF16, bias=fx.bias)
+        assert float(np.linalg.norm(got - ref) / np.linalg.norm(ref)) < 1e-6
+    mlxq.streamStatus(None, 0)
+
+
+def test_full_precision_gemm_in_slices_of_tokens(mlxq, oracle):
+    # 12288 fp32 codes a token on five row tiles: a slice holds 1408 tokens (scratch for both parts and eight sums an output), so 4500 tokens
+    # take several turns over the same scratch memory, the last one shorter.  Tokens on both sides of every multiple of 128 that may
+    # be a boundary against the oracle, and every token against the same one in a short batch, bit for bit.
+    O, K, T = 520, 12288, 4500
+    fx = oracle.QuantFixture(O=O, K=K, bits=8, gs=64, scale_type=oracle.BF16, seed=3)
+    layer = DevLayer.from_fixture(mlxq, fx)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1)
+    x = torch.rand((T, K), device="cuda", generator=gen) * 2 - 1
+    y, part = torch.full((T, O), float("nan"), device="cuda"), torch.full((T, O), float("nan"), device="cuda")
+    layer.linear.encode(None, x, K, y, O, T)
+    for t0 in range(0, T, 100):
+        layer.linear.encode(None, x[t0:], K, part[t0:], O, min(100, T - t0))
+    torch.cuda.synchronize()
+    mlxq.streamStatus(None, 0)
+    assert torch.equal(y, part)
+    tokens = [t for b in range(0, T, 128) for t in (b - 1, b) if 0 <= t < T] + [T - 1]
+    ref = _ref(oracle, fx, x[tokens].cpu().numpy(), K, 8, 64, oracle.BF16)
+    assert float(np.linalg.norm(y[tokens].cpu().numpy() - ref) / np.linalg.norm(ref)) < 1e-6
+
+
+@pytest.mark.parametrize("T", [17, 77, 128])
+def test_tall_tile_of_short_batches_on_many_rows(mlxq, oracle, T):
+    # more row tiles than one round of the SMs holds, at most 128 tokens: 256 rows a tile, the last one ragged.  The same tokens
+    # in a batch of 256 take the wide tile: the sums are the same, bit for bit.
+    O, K = 19001, 512
+    fx = oracle.QuantFixture(O=O, K=K, bits=4, gs=64, scale_type=oracle.BF16, with_bias=True, seed=T)
+    layer = DevLayer.from_fixture(mlxq, fx)
+    assert layer.linear.gemmTileTokens(T) == 128
+    x = oracle.RNG(T).floats(256 * K).reshape(256, K)
+    xr = as_dtype(x, 2).float().cpu().numpy()
+    got, wide = run(layer, x[:T], T, x_dtype=2, y_stride=O + 3), run(layer, x, 256, x_dtype=2)
+    mlxq.streamStatus(None, 0)
+    assert np.array_equal(got.view(np.uint32), wide[:T].view(np.uint32))
+    rows = np.r_[0:130, 9000:9300, 18900:O]
+    ref = _sampled(oracle, fx, xr, rows, np.arange(T)) + fx.bias[rows]
+    assert float(np.linalg.norm(got[:, rows] - ref) / np.linalg.norm(ref)) < 5e-4

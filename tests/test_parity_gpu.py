@@ -181,9 +181,11 @@ def test_small_batches_every_width_and_group(mlxq, oracle, bits):
 
 @pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
 def test_small_batches_of_long_rows(mlxq, oracle, bits):
-    # rows of 6144 codes and more are split over the CTAs of a cluster: even and uneven slices, fewer blocks than clusters
-    # and several rounds of them, 16 tokens of 16-bit activations (a wider cluster where the slices do not fit)
-    for gs, K, O, T, x_dtype in ((64, 6144, 41, 2, 0), (32, 6656, 600, 6, 0), (128, 12288, 24, 8, 0), (64, 14336, 40, 16, 1), (64, 6400, 700, 5, 2)):
+    # rows of 6144 codes and more: single CTAs, and clusters where those do not hold the tokens -- even and uneven slices, fewer
+    # blocks than clusters and several rounds of them, 16 tokens of 16-bit activations (a wider cluster where the slices do not
+    # fit)
+    for gs, K, O, T, x_dtype in ((64, 6144, 41, 2, 0), (32, 6656, 600, 6, 0), (128, 12288, 24, 8, 0), (64, 14336, 40, 16, 1), (64, 6400, 700, 5, 2),
+                                (64, 6144, 700, 8, 0), (64, 12288, 600, 6, 0), (64, 6144, 41, 16, 1), (128, 14336, 600, 10, 2)):
         fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=gs, scale_type=oracle.BF16, with_bias=(gs == 64), seed=bits + K)
         layer = DevLayer.from_fixture(mlxq, fx)
         x = oracle.RNG(T + K + bits).floats(T * K).reshape(T, K)
