@@ -41,7 +41,7 @@ PASSES = 48          # passes per step: 768 launches, ~6 ms of device time
 # DRAM bytes one launch of the decode kernel moved in an ncu capture of this workload's kernel at this shape
 # (dram__bytes_read.sum + dram__bytes_write.sum); reported as roofline.traffic for that shape on one GPU only.
 NCU_DRAM_BYTES_PER_LAUNCH = 25403904
-NCU_TRAFFIC_SOURCE = "ncu capture summarised in profiles/qmv_pipe_b4g64_m1.md (not measured in this run)"
+NCU_TRAFFIC_SOURCE = "ncu capture of this kernel at this shape (not measured in this run)"
 METRIC = "decode_qmv_hbm_gbs"
 UNIT = "GB/s"
 

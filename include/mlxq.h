@@ -139,7 +139,8 @@ MLXQ_API int mlxq_linear_forward(mlxq_linear_t h, mlxq_stream_t stream, const vo
  *     rounded up to 256), are rejected with MLXQ_INVALID_ARGUMENT (split the batch; shard the layer).
  *   - Batches the 4-bit GEMM does not take (T <= 16, fp32 activations, other bit widths) run on kernels that use no
  *     scratch memory.  Beyond 16 tokens mlxq_linear_forward has a GEMM for them that does (and is much faster): there
- *     the two agree to the fp32 rounding of their sums, not bit for bit.  The same holds between a batch encoded while
+ *     the two agree to the fp32 rounding of their sums, not bit for bit,
+ *     for activations that fp16 numbers hold (the GEMM scales others, most of these kernels do not).  The same holds between a batch encoded while
  *     its stream is captured, which keeps these kernels, and one that is not.
  *   - Every call on a device shares the one array, which keeps whatever the last call wrote: calls that
  *     overlap on the GPU (different streams) race; order them on one stream or with events.

@@ -1,5 +1,5 @@
-// Prefill GEMM for sm_100a at the precision of the decode kernels: Y[T, O] = X[T, K] . W[O, K]^T, any MLX bit width,
-// fp32 / fp16 / bf16 activations, scales, biases and sums over groups in fp32.
+// Prefill GEMM for sm_100a that rounds no operand to fp16's 11 bits or range: Y[T, O] = X[T, K] . W[O, K]^T, any MLX bit
+// width, fp32 / fp16 / bf16 activations of any magnitude, scales, biases and sums over groups in fp32.
 //
 // What it replaces: batches whose weights or activations may not be rounded to fp16 (everything but 4-bit layers with
 // 16-bit activations) ran eight or sixteen tokens at a time on the token-major decode kernel, or on the CUDA cores when

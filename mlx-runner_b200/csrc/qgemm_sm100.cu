@@ -62,7 +62,8 @@ constexpr int W_PRODUCER = 2;           // warp that streams the packed weight s
 // Two warps issue the MMAs, one per 128-row half of the tile.  From a branch that lane 0 takes alone an MMA cost ~110
 // cycles to issue (its operands travel through uniform registers) while an M128 N128 K16 MMA executes in 64.  The lanes
 // now stay together and elect one for the instruction, and one poll serves both barriers of a stage: 12288 x 4096 with
-// 1999 tokens 210.9 -> 198.2 us, 14336 x 4096 with 8192 tokens 880 -> 846 us.  The halves use separate accumulators and separate A
+// 1999 tokens 210.9 -> 198.2 us (at the power cap, 14336 x 4096 with 8192 tokens, about 2 % of 1000 us).  The halves use separate
+// accumulators and separate A
 // columns, so nothing orders the two issuers against each other; stage and accumulator barriers count both.
 constexpr int MMA_WARP = 1;             // issuer of half 0; it also owns the tensor-memory allocation
 constexpr int MMA_WARP2 = 3;            // issuer of half 1
