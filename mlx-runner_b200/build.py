@@ -28,12 +28,14 @@ COMMON = ARCH + ["-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcom
                  "--expt-relaxed-constexpr", "-I", os.path.join(ROOT, "include")]
 
 # (source, object name, extra flags)
-UNITS = [("qmv_inst.cu", f"qmv_b{b}.o", [f"-DMLXQ_BITS={b}"]) for b in (2, 3, 4, 5, 6, 8)] + [
+UNITS = [("qmv_inst.cu", f"qmv_b{b}.o", [f"-DMLXQ_BITS={b}"]) for b in (2, 3, 4, 5, 6, 8)] + \
+        [("qmv_tc_inst.cu", f"qmv_tc_b{b}.o", [f"-DMLXQ_BITS={b}"]) for b in (2, 3, 4, 5, 6, 8)] + [
     ("aux_kernels.cu", "aux_kernels.o", []),
     ("dense.cu", "dense.o", []),
     ("qmv_mma.cu", "qmv_mma.o", []),
     ("qmv_pipe.cu", "qmv_pipe.o", []),
     ("qmv_tok.cu", "qmv_tok.o", []),
+    ("qmv_tc.cu", "qmv_tc.o", []),
     ("qgemm_sm100.cu", "qgemm_sm100.o", []),
     ("qgemm_exact.cu", "qgemm_exact.o", []),
     ("api.cu", "api.o", []),

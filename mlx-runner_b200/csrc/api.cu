@@ -20,6 +20,7 @@
 #include "qmv_pipe.cuh"
 #include "dense.cuh"
 #include "qmv_tok.cuh"
+#include "qmv_tc.cuh"
 
 namespace mlxq {
 
@@ -281,6 +282,20 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
                 if (rc != MLXQ_OK) return rc;
             }
             return MLXQ_OK;
+        }
+    }
+    if (T >= 2 && T <= 16 && !getenv("MLXQ_DECODE")) {
+        // small batches: the tensor-memory kernel where it serves the call and is the faster one (MLXQ_DECODE names the others)
+        MmaParams mt = {};
+        p.T = static_cast<int>(T); p.x = x; p.y = y;
+        mt.q = p;
+        mt.split = x_dtype == MLXQ_F32 ? 2 : 1;
+        mt.err = device_error_word(parts[0]->device);
+        TcPlan tc;
+        const size_t tsmem = mt.err ? qmv_tc_plan(parts[0]->bits, mt, static_cast<int>(T), tc) : 0;
+        if (tsmem) {
+            const cudaError_t err = launch_qmv_tc(parts[0]->bits, mt, tc, tsmem, parts[0]->device, st);
+            return err == cudaSuccess ? MLXQ_OK : cuda_fail(err, "qmv (tensor memory) launch");
         }
     }
     MmaParams mp;
