@@ -52,6 +52,10 @@ template <int BITS> __device__ __forceinline__ int stage_shift(int i) {
     return 0;
 }
 
+// Rows beyond this length are planned by no kernel that stages activations in shared memory: at two bytes a code or more the eight
+// CTAs of the largest cluster hold 917,504 of them.  The planners refuse them first, so that their sizes stay far inside 32 bits.
+constexpr int STAGED_K_MAX = 1 << 20;
+
 struct MmaParams {
     QmvParams q;            // layer parts, x, y, strides, dtypes, epilogue
     int xn;                 // staged activation columns: tokens, or 2 * tokens for fp32 activations

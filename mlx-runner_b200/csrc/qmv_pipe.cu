@@ -84,7 +84,7 @@ cudaError_t launch_bits(const MmaParams& p, const PipePlan& pp, size_t smem, int
 
 size_t qmv_pipe_plan(int bits, const MmaParams& p, int tokens, int sms, PipePlan& pp) {
     const QmvParams& q = p.q;
-    if (p.passes > 4 || tokens < 1 || q.total_rows < 1) return 0;
+    if (q.K > STAGED_K_MAX || p.passes > 4 || tokens < 1 || q.total_rows < 1) return 0;
     int lb, kb;
     unit_for(bits, lb, kb);
     const int K = q.K, groups = K / q.gs;

@@ -126,7 +126,7 @@ int k_split(int n_blocks) { return n_blocks <= 1024 ? 4 : 2; }
 
 size_t qmv_tok_plan(int bits, const MmaParams& p, int tokens, int sms, TokPlan& tp, int clusters) {
     const QmvParams& q = p.q;
-    if (tokens < 1 || q.total_rows < 1 || p.xn < 1 || p.xn > 16) return 0;
+    if (q.K > STAGED_K_MAX || tokens < 1 || q.total_rows < 1 || p.xn < 1 || p.xn > 16) return 0;
     if (q.gs != 32 && q.gs != 64 && q.gs != 128) return 0;
     if (!supported(bits, q.gs)) return 0;
     if (q.s_dtype != DT_F16 && q.s_dtype != DT_BF16) return 0;     // a 16-bit bias is exact in TF32; an fp32 one is not

@@ -1,0 +1,61 @@
+"""The decode kernels' planners, run on the host: what they place lies inside the shared memory they ask for."""
+import importlib.util
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+PKG = os.path.join(ROOT, "mlx-runner_b200")
+
+SMEM_OPT_IN = 227 * 1024
+
+
+@pytest.fixture(scope="module")
+def plans(tmp_path_factory):
+    """calls -> planned layouts: lists of integers, one per planner (see decode_plans.cu)."""
+    spec = importlib.util.spec_from_file_location("mlxq_build", os.path.join(PKG, "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    build.build()
+    exe = str(tmp_path_factory.mktemp("plans") / "decode_plans")
+    objs = [os.path.join(build.OBJ, o) for (_, o, _) in build.UNITS]
+    subprocess.run([build._nvcc()] + build.COMMON + ["-I", build.CSRC, os.path.join(HERE, "decode_plans.cu"), "-o", exe] + objs + ["-ldl"], check=True)
+
+    def run(calls):
+        text = "\n".join(" ".join(str(v) for v in c) for c in calls)
+        out = subprocess.run([exe], input=text, capture_output=True, text=True, check=True).stdout.splitlines()
+        assert len(out) == len(calls)
+        return [[[int(v) for v in part.split()] for part in line.split("|")] for line in out]
+
+    return run
+
+
+def test_no_row_length_leaves_the_shared_memory_asked_for(plans):
+    # a layer may have rows of up to 2^30 codes: lengths at which a 32-bit size of 2, 4, 8 ... 64 bytes a code wraps around,
+    # lengths around them, and a walk over the rest
+    lengths = {65075328, 33554432, 1 << 30}
+    for shift in range(20, 31):
+        for num in range(1, 16):
+            at = (num << shift) // 4
+            lengths.update(at + d * 128 for d in (-80, -3, -1, 0, 1, 2, 40) if 1024 <= at + d * 128 <= 1 << 30)
+    lengths.update(range(1024, 1 << 18, 640))
+    lengths.update(range(1 << 18, 1 << 30, 1021 * 1024))
+    calls = [(bits, gs, k // 128 * 128, rows, tokens, split) for k in sorted(lengths)
+             for bits, gs, rows, tokens, split in ((4, 64, 128, 16, 2), (8, 32, 40, 8, 2), (4, 128, 4096, 16, 1), (2, 64, 24, 3, 2), (6, 32, 64, 6, 2))]
+    served = 0
+    for call, (tc, *others) in zip(calls, plans(calls)):
+        smem, kz, stages, depth, off_x, off_xsum, off_red, off_bars = tc
+        if smem:
+            served += 1
+            bits, gs, k, rows, tokens, split = call
+            slice_ = -(-stages // kz)
+            x_bytes = slice_ * 2 * split * (1024 if tokens <= 8 else 2048)
+            assert stages == k // 128 and depth >= 3 and smem <= SMEM_OPT_IN, call
+            assert 0 < off_x and off_x + x_bytes <= off_xsum < off_red < off_bars < smem, f"{call}: {tc}"
+        for plan in others:
+            if plan[0]:
+                served += 1
+                assert plan[0] <= SMEM_OPT_IN and all(a <= b for a, b in zip([1] + plan[1:], plan[1:] + [plan[0]])), f"{call}: {plan}"
+    assert served > 300
