@@ -220,14 +220,23 @@ static void fill_qmv(QmvParams& p, const mlxq_linear_t* parts, int n) {
     for (int s = 3; s < 31; s++) if ((1 << s) == f->gs) p.gs_shift = s;
 }
 
+// The decode kernel that MLXQ_DECODE names: cuda, mma, pipe, tok (the dispatch without the tensor-memory kernel) or tc (that
+// kernel wherever it can serve a call).  Anything else names none.
+enum class Decode { any, cuda, mma, pipe, tok, tc };
+static Decode decode_named() {
+    const char* mode = getenv("MLXQ_DECODE");
+    if (!mode) return Decode::any;
+    return strcmp(mode, "cuda") == 0 ? Decode::cuda : strcmp(mode, "mma") == 0 ? Decode::mma : strcmp(mode, "pipe") == 0 ? Decode::pipe :
+           strcmp(mode, "tok") == 0 ? Decode::tok : strcmp(mode, "tc") == 0 ? Decode::tc : Decode::any;
+}
+
 // The tensor-core decode kernel takes a call when the batch is small, the group size is 32/64/128, K is a
 // multiple of the kernel's step and the rows are aligned for vector loads.  MLXQ_DECODE=cuda forces the
 // CUDA-core kernel (which handles every shape).  Returns the shared memory needed, 0 when not eligible.
 static size_t mma_plan(const mlxq_linear_t* parts, int n, int x_dtype, int64_t T, MmaParams& mp, bool* planned = nullptr) {
     if (planned) *planned = false;
     const mlxq_linear* f = parts[0];
-    const char* mode = getenv("MLXQ_DECODE");
-    if (mode && strcmp(mode, "cuda") == 0) return 0;
+    if (decode_named() == Decode::cuda) return 0;
     if (T > 16 || (f->gs != 32 && f->gs != 64 && f->gs != 128)) return 0;
     const int kb = qmv_mma_step_codes(f->bits);
     if (f->in_dim % kb != 0) return 0;
@@ -255,6 +264,7 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
     p.y_stride = y_stride;
     p.e = e;
     p.act = act;
+    const Decode mode = decode_named();
     if (T > 16 && !peer && !x_up && !e) {
         // A long batch that neither tensor-core GEMM takes (or that must not use scratch memory): sixteen (or eight)
         // tokens at a time on the token-major kernel -- the weights are then read once per sixteen tokens through
@@ -268,8 +278,7 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
             mc.q = p;
             mc.err = device_error_word(parts[0]->device);
             TokPlan tc;
-            const char* mode = getenv("MLXQ_DECODE");
-            if (!mc.err || (mode && (strcmp(mode, "mma") == 0 || strcmp(mode, "pipe") == 0)) ||
+            if (!mc.err || mode == Decode::mma || mode == Decode::pipe ||
                 !qmv_tok_plan(parts[0]->bits, mc, chunk, device_sm_count(parts[0]->device), tc))
                 continue;
             // (every call takes exactly `chunk` tokens -- the last one reaches back over tokens already done -- so a token's
@@ -284,15 +293,15 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
             return MLXQ_OK;
         }
     }
-    if (T >= 2 && T <= 16 && !getenv("MLXQ_DECODE")) {
-        // small batches: the tensor-memory kernel where it serves the call and is the faster one (MLXQ_DECODE names the others)
+    if (T >= 2 && T <= 16 && (mode == Decode::any || mode == Decode::tc)) {
+        // small batches: the tensor-memory kernel where it serves the call and is the faster one
         MmaParams mt = {};
         p.T = static_cast<int>(T); p.x = x; p.y = y;
         mt.q = p;
         mt.split = x_dtype == MLXQ_F32 ? 2 : 1;
         mt.err = device_error_word(parts[0]->device);
         TcPlan tc;
-        const size_t tsmem = mt.err ? qmv_tc_plan(parts[0]->bits, mt, static_cast<int>(T), tc) : 0;
+        const size_t tsmem = mt.err ? qmv_tc_plan(parts[0]->bits, mt, static_cast<int>(T), mode == Decode::tc, tc) : 0;
         if (tsmem) {
             const cudaError_t err = launch_qmv_tc(parts[0]->bits, mt, tc, tsmem, parts[0]->device, st);
             return err == cudaSuccess ? MLXQ_OK : cuda_fail(err, "qmv (tensor memory) launch");
@@ -308,9 +317,8 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
         mp.q = p;
         mp.err = device_error_word(parts[0]->device);
         // Preferred: the persistent kernel fed by asynchronous copies (MLXQ_DECODE=mma keeps the register-fed one).
-        const char* mode = getenv("MLXQ_DECODE");
-        const bool persistent = !(mode && strcmp(mode, "mma") == 0) && mp.err;
-        if (persistent && T >= 2 && !(mode && strcmp(mode, "pipe") == 0)) {
+        const bool persistent = mode != Decode::mma && mp.err;
+        if (persistent && T >= 2 && mode != Decode::pipe) {
             // two or more tokens: the token-major kernel where it serves the call (MLXQ_DECODE=pipe keeps the other)
             TokPlan tp;
             const size_t tsmem = qmv_tok_plan(parts[0]->bits, mp, static_cast<int>(T), device_sm_count(parts[0]->device), tp);
@@ -348,7 +356,7 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
         // fits some three-token calls, 1.15 at 6 bits).  4096 x 14336, 3 fp32 tokens, 4 bits: 240 -> 24 us.
         const int bits = parts[0]->bits;
         const bool as_exact = bits <= 5 || (bits == 6 && !smem) || (bits == 8 && mp.split == 2);
-        if (persistent && !rsmem && T >= 2 && !(mode && strcmp(mode, "pipe") == 0) && (fit == 4 || peer || (!fit && (as_exact || x_up)))) {
+        if (persistent && !rsmem && T >= 2 && mode != Decode::pipe && (fit == 4 || peer || (!fit && (as_exact || x_up)))) {
             TokPlan tp;
             const size_t tsmem = qmv_tok_plan(bits, mp, static_cast<int>(T), device_sm_count(parts[0]->device), tp, fit == 4 ? 1 : 2);
             if (tsmem) {
@@ -414,7 +422,7 @@ static int gemm_tile_for(const mlxq_linear* h, int x_dtype, int64_t x_stride, co
 // memory would become allocation nodes of the caller's graph, where the kernels of run_qmv leave plain kernel nodes.
 // MLXQ_DECODE names one of those kernels and is obeyed.
 static bool exact_gemm_for(const mlxq_linear* h, int x_dtype, int64_t x_stride, const void* x, int64_t T, cudaStream_t st) {
-    if (T < 17 || T < gemm_min_tokens() || h->bits == 0 || getenv("MLXQ_DECODE") || !qgemm_exact_takes(gemm_layer(h), x_dtype, x_stride, x, T))
+    if (T < 17 || T < gemm_min_tokens() || h->bits == 0 || decode_named() != Decode::any || !qgemm_exact_takes(gemm_layer(h), x_dtype, x_stride, x, T))
         return false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;

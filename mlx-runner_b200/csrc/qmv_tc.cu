@@ -43,11 +43,11 @@ bool worth(int bits, int gs, int K, int rows, int tokens, int split) {
 
 }  // namespace
 
-size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, TcPlan& tp) {
+size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, bool always, TcPlan& tp) {
     const QmvParams& q = p.q;
     if (q.K > STAGED_K_MAX || tokens < 2 || tokens > 16 || q.peer.n > 0 || q.x_up != nullptr || q.e != nullptr) return 0;
     if ((q.gs != 32 && q.gs != 64 && q.gs != 128) || (q.s_dtype != DT_F16 && q.s_dtype != DT_BF16) || q.K % TC_STAGE != 0) return 0;
-    if (!worth(bits, q.gs, q.K, q.total_rows, tokens, p.split)) return 0;
+    if (!always && !worth(bits, q.gs, q.K, q.total_rows, tokens, p.split)) return 0;
     tp = TcPlan{};
     uintptr_t at = 16;
     for (int i = 0; i < q.n_parts; i++) {

@@ -9,8 +9,8 @@
 using namespace mlxq;
 
 int main() {
-    int bits, gs, K, rows, tokens, split;
-    while (std::scanf("%d %d %d %d %d %d", &bits, &gs, &K, &rows, &tokens, &split) == 6) {
+    int bits, gs, K, rows, tokens, split, always;
+    while (std::scanf("%d %d %d %d %d %d %d", &bits, &gs, &K, &rows, &tokens, &split, &always) == 7) {
         MmaParams p = {};
         QmvParams& q = p.q;
         for (QmvPart& part : q.part) {
@@ -28,7 +28,7 @@ int main() {
         for (int s = 3; s < 31; s++) if ((1 << s) == gs) q.gs_shift = s;
         p.split = split;
         TcPlan tc = {};
-        const size_t tcs = qmv_tc_plan(bits, p, tokens, tc);
+        const size_t tcs = qmv_tc_plan(bits, p, tokens, always != 0, tc);
         std::printf("%zu %d %d %d %d %d %d %d", tcs, tc.kz, tc.stages, tc.depth, tc.off_x, tc.off_xsum, tc.off_red, tc.off_bars);
         const bool columns = qmv_mma_plan(bits, K, gs, tokens * split, p);
         for (int clusters = 0; clusters <= 2; clusters++) {

@@ -42,14 +42,14 @@ def test_no_row_length_leaves_the_shared_memory_asked_for(plans):
             lengths.update(at + d * 128 for d in (-80, -3, -1, 0, 1, 2, 40) if 1024 <= at + d * 128 <= 1 << 30)
     lengths.update(range(1024, 1 << 18, 640))
     lengths.update(range(1 << 18, 1 << 30, 1021 * 1024))
-    calls = [(bits, gs, k // 128 * 128, rows, tokens, split) for k in sorted(lengths)
+    calls = [(bits, gs, k // 128 * 128, rows, tokens, split, 1) for k in sorted(lengths)
              for bits, gs, rows, tokens, split in ((4, 64, 128, 16, 2), (8, 32, 40, 8, 2), (4, 128, 4096, 16, 1), (2, 64, 24, 3, 2), (6, 32, 64, 6, 2))]
     served = 0
     for call, (tc, *others) in zip(calls, plans(calls)):
         smem, kz, stages, depth, off_x, off_xsum, off_red, off_bars = tc
         if smem:
             served += 1
-            bits, gs, k, rows, tokens, split = call
+            bits, gs, k, rows, tokens, split, _ = call
             slice_ = -(-stages // kz)
             x_bytes = slice_ * 2 * split * (1024 if tokens <= 8 else 2048)
             assert stages == k // 128 and depth >= 3 and smem <= SMEM_OPT_IN, call

@@ -1,0 +1,36 @@
+"""Calls of two to sixteen tokens have two kernels, the token-major one (qmv_tok.cuh) and the tensor-memory one (qmv_tc.cuh):
+which of them takes a call, and the tensor-memory kernel at its edges, against the oracle.  MLXQ_DECODE is read at every call."""
+import pytest
+import torch
+
+from helpers import DevLayer, as_dtype
+
+pytestmark = pytest.mark.gpu
+
+
+def forward(layer, x, T):
+    O = layer.linear.outDim
+    y = torch.full((T, O), float("nan"), device="cuda")
+    layer.linear.encode(None, x, layer.linear.inDim, y, O, T)
+    torch.cuda.synchronize()
+    return y
+
+
+def test_a_kernel_is_chosen_by_its_name_only(mlxq, oracle, monkeypatch):
+    # 12 fp32 tokens: the tensor-memory kernel's; a value that names no kernel changes nothing
+    K, O, T = 2048, 264, 12
+    fx = oracle.QuantFixture(O=O, K=K, bits=4, gs=64, scale_type=oracle.BF16, seed=3)
+    layer = DevLayer.from_fixture(mlxq, fx)
+    x = as_dtype(oracle.RNG(5).floats(T * K).reshape(T, K), 0)
+    got = {}
+    for mode in (None, "", "another", "tc", "tok", "cuda"):
+        if mode is None:
+            monkeypatch.delenv("MLXQ_DECODE", raising=False)
+        else:
+            monkeypatch.setenv("MLXQ_DECODE", mode)
+        got[mode] = forward(layer, x, T)
+    for mode in ("", "another", "tc"):
+        assert torch.equal(got[mode], got[None]), f"MLXQ_DECODE={mode!r} changed the kernel"
+    for mode in ("tok", "cuda"):
+        assert not torch.equal(got[mode], got[None]), f"MLXQ_DECODE={mode!r} was not obeyed"
+        assert oracle.max_rel_err(got[mode].cpu().numpy(), fx.reference(x.cpu().numpy())) < 1e-4
