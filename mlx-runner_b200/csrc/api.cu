@@ -293,7 +293,11 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
             return MLXQ_OK;
         }
     }
-    if (T >= 2 && T <= 16 && (mode == Decode::any || mode == Decode::tc)) {
+    // (A shard keeps to the kernels that can store into the peers' windows, so that its rows are the same bits whichever way they
+    // are gathered.)
+    bool sharded = false;
+    for (int i = 0; i < n; i++) sharded = sharded || parts[i]->shard_count > 1;
+    if (T >= 2 && T <= 16 && !sharded && (mode == Decode::any || mode == Decode::tc)) {
         // small batches: the tensor-memory kernel where it serves the call and is the faster one
         MmaParams mt = {};
         p.T = static_cast<int>(T); p.x = x; p.y = y;

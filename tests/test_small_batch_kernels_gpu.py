@@ -34,3 +34,26 @@ def test_a_kernel_is_chosen_by_its_name_only(mlxq, oracle, monkeypatch):
     for mode in ("tok", "cuda"):
         assert not torch.equal(got[mode], got[None]), f"MLXQ_DECODE={mode!r} was not obeyed"
         assert oracle.max_rel_err(got[mode].cpu().numpy(), fx.reference(x.cpu().numpy())) < 1e-4
+
+
+@pytest.mark.parametrize("x_dtype,T", [(0, 4), (0, 8), (0, 12), (2, 13)])
+def test_shards_keep_to_the_kernels_of_the_fused_gather(mlxq, oracle, monkeypatch, x_dtype, T):
+    # the fused gather runs on the token-major kernel (or what stands in for it), the gathers after the call must give the
+    # same bits: rows of 4096 codes, where a whole layer's batches take the tensor-memory kernel
+    K, O, bits, gs = 4096, 1024, 4, 64
+    fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=gs, scale_type=oracle.BF16, seed=T)
+    full = DevLayer.from_fixture(mlxq, fx)
+    shard = mlxq.Linear.shard(full.w, full.s, full.b, None, inDim=K, rank=1, nranks=2, full=True, name="shard", device=0)
+    x = as_dtype(oracle.RNG(T).floats(T * K).reshape(T, K), x_dtype)
+    got = {}
+    for mode in (None, "tok"):
+        if mode is None:
+            monkeypatch.delenv("MLXQ_DECODE", raising=False)
+        else:
+            monkeypatch.setenv("MLXQ_DECODE", mode)
+        y = torch.full((T, O // 2), float("nan"), device="cuda")
+        shard.encode(None, x, K, y, O // 2, T)
+        torch.cuda.synchronize()
+        got[mode] = y
+    assert torch.equal(got[None], got["tok"])
+    assert oracle.max_rel_err(got[None].cpu().numpy(), fx.reference(x.float().cpu().numpy())[:, O // 2:]) < 1e-3
