@@ -3,7 +3,7 @@ which of them takes a call, and the tensor-memory kernel at its edges, against t
 import pytest
 import torch
 
-from helpers import DevLayer, as_dtype
+from helpers import TORCH_DT, DevLayer, as_dtype
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +57,38 @@ def test_shards_keep_to_the_kernels_of_the_fused_gather(mlxq, oracle, monkeypatc
         got[mode] = y
     assert torch.equal(got[None], got["tok"])
     assert oracle.max_rel_err(got[None].cpu().numpy(), fx.reference(x.float().cpu().numpy())[:, O // 2:]) < 1e-3
+
+
+def codes_of(w, bits, K):
+    """Packed words -> codes [rows, K]"""
+    b = w.view(torch.uint8).view(w.shape[0], -1)
+    if bits in (2, 4, 8):
+        return torch.stack([(b >> at) & ((1 << bits) - 1) for at in range(0, 8, bits)], -1).reshape(-1, K)
+    one = torch.stack([(b >> i) & 1 for i in range(8)], -1).reshape(-1, K, bits)
+    return (one << torch.arange(bits, dtype=torch.uint8, device=w.device)).sum(-1, dtype=torch.uint8)
+
+
+@pytest.mark.parametrize("bits,gs,K,O,T,x_dtype", [(8, 32, 12288, 512, 16, 2), (8, 32, 14336, 512, 11, 1), (8, 64, 12288, 8192, 13, 2),
+                                                   (6, 32, 12288, 512, 13, 2), (5, 32, 14336, 512, 5, 2), (4, 64, 4096, 512, 6, 0), (8, 128, 12288, 512, 16, 1)])
+def test_no_less_exact_than_the_kernels_before(mlxq, monkeypatch, bits, gs, K, O, T, x_dtype):
+    # the error against 64 bits, with the kernel that the dispatch takes and without the tensor-memory kernel.  A norm over
+    # O * T >= 2560 outputs with independent roundings is known to 1 / sqrt(2 * 2560) = 1.4 %: three times that.
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(K + T)
+    w = torch.randint(-(1 << 31), (1 << 31) - 1, (O, K * bits // 32), dtype=torch.int32, device="cuda", generator=gen)
+    s = (torch.randn((O, K // gs), device="cuda", generator=gen).abs() * 0.002 + 1e-4).to(torch.bfloat16)
+    b = (-float(1 << (bits - 1)) * s.float()).to(torch.bfloat16)
+    lin = mlxq.Linear(w, s, b, None, inDim=K)
+    x = torch.randn((T, K), device="cuda", generator=gen).to(TORCH_DT[x_dtype])
+    ref = x.double() @ (codes_of(w, bits, K).double() * s.double().repeat_interleave(gs, 1) + b.double().repeat_interleave(gs, 1)).T
+    err = {}
+    for mode in (None, "tok"):
+        if mode is None:
+            monkeypatch.delenv("MLXQ_DECODE", raising=False)
+        else:
+            monkeypatch.setenv("MLXQ_DECODE", mode)
+        y = torch.full((T, O), float("nan"), device="cuda")
+        lin.encode(None, x, K, y, O, T)
+        torch.cuda.synchronize()
+        err[mode] = ((y.double() - ref).norm() / ref.norm()).item()
+    assert err[None] <= 1.05 * err["tok"], err
