@@ -305,7 +305,7 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
         mt.split = x_dtype == MLXQ_F32 ? 2 : 1;
         mt.err = device_error_word(parts[0]->device);
         TcPlan tc;
-        const size_t tsmem = mt.err ? qmv_tc_plan(parts[0]->bits, mt, static_cast<int>(T), mode == Decode::tc, tc) : 0;
+        const size_t tsmem = mt.err ? qmv_tc_plan(parts[0]->bits, mt, static_cast<int>(T), mode == Decode::tc, qmv_tc_room(parts[0]->device, device_sm_count(parts[0]->device)), tc) : 0;
         if (tsmem) {
             const cudaError_t err = launch_qmv_tc(parts[0]->bits, mt, tc, tsmem, parts[0]->device, st);
             return err == cudaSuccess ? MLXQ_OK : cuda_fail(err, "qmv (tensor memory) launch");

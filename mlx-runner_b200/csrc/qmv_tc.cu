@@ -1,7 +1,12 @@
 // Planner and launcher of the tensor-memory decode matvec (qmv_tc.cuh).
 #include "qmv_tc.cuh"
 
+#include <mutex>
+
 namespace mlxq {
+
+// (qmv_tc_inst.cu) clusters of `kz` CTAs with `smem` bytes each that the current device holds at once; 0 where it cannot say
+int qmv_tc_clusters(int kz, size_t smem);
 
 cudaError_t launch_qmv_tc_b2(const MmaParams&, const TcPlan&, size_t, int, cudaStream_t);
 cudaError_t launch_qmv_tc_b3(const MmaParams&, const TcPlan&, size_t, int, cudaStream_t);
@@ -43,7 +48,24 @@ bool worth(int bits, int gs, int K, int rows, int tokens, int split) {
 
 }  // namespace
 
-size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, bool always, TcPlan& tp) {
+// Asked for once per device, with that device current.  (B200: 148 SMs, 148, 74, 33 and 15 clusters with one CTA an SM, 296, 148,
+// 71 and 33 with two: parts of the chip have an SM count that is no multiple of the cluster's.)
+const TcRoom& qmv_tc_room(int device, int sms) {
+    static std::mutex mu;
+    static TcRoom rooms[64] = {};
+    TcRoom& r = rooms[device];
+    std::lock_guard<std::mutex> lk(mu);
+    if (r.sms == 0) {
+        for (int shift = 0; shift <= 3; shift++) {
+            r.one[shift] = qmv_tc_clusters(1 << shift, TC_SMEM_WHOLE);
+            r.two[shift] = qmv_tc_clusters(1 << shift, TC_SMEM_TWO);
+        }
+        r.sms = sms;
+    }
+    return r;
+}
+
+size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, bool always, const TcRoom& room, TcPlan& tp) {
     const QmvParams& q = p.q;
     if (q.K > STAGED_K_MAX || tokens < 2 || tokens > 16 || q.peer.n > 0 || q.x_up != nullptr || q.e != nullptr) return 0;
     if ((q.gs != 32 && q.gs != 64 && q.gs != 128) || (q.s_dtype != DT_F16 && q.s_dtype != DT_BF16) || q.K % TC_STAGE != 0) return 0;
@@ -82,11 +104,10 @@ size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, bool always, TcPlan
         int depth = ((two ? TC_SMEM_TWO : TC_SMEM_WHOLE) - fixed) / slot;
         if (depth < 3) continue;
         depth = depth >= 8 ? 8 : depth >= 6 ? 6 : depth >= 4 ? 4 : 3;
-        // clusters that a B200's 148 SMs hold at once (as cudaOccupancyMaxActiveClusters says)
-        constexpr int by_two[4] = {296, 148, 71, 33}, by_one[4] = {148, 74, 33, 15};
-        const int resident = (two ? by_two : by_one)[shift], clusters = tp.n_blocks < resident ? tp.n_blocks : resident;
+        const int resident = (two ? room.two : room.one)[shift], clusters = tp.n_blocks < resident ? tp.n_blocks : resident;
+        if (clusters < 1) continue;
         const int rounds = (tp.n_blocks + clusters - 1) / clusters;
-        const double cost = rounds * (slice * (clusters * kz > 148 ? 0.8 : 0.47) + 2.0);
+        const double cost = rounds * (slice * (clusters * kz > room.sms ? 0.8 : 0.47) + 2.0);
         if (best_smem != 0 && cost >= best) continue;
         best = cost;
         tp.kz = kz; tp.kz_shift = shift; tp.clusters = clusters; tp.depth = depth;

@@ -622,9 +622,16 @@ qmv_tc_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TcPla
     if (kz > 1) tc_cluster_barrier();                           // nobody leaves while others store into its shared memory or arrive there
 }
 
+// What a device holds at once: its SMs, and clusters of 1, 2, 4 and 8 CTAs with one CTA an SM and with two.
+struct TcRoom {
+    int sms;
+    int one[4], two[4];
+};
+const TcRoom& qmv_tc_room(int device, int sms);
+
 // Plans a call; returns the shared memory it needs, 0 when the call is not one the kernel serves or, unless `always`, not one
 // that it is the faster for.
-size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, bool always, TcPlan& tp);
+size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, bool always, const TcRoom& room, TcPlan& tp);
 cudaError_t launch_qmv_tc(int bits, const MmaParams& p, const TcPlan& tp, size_t smem, int device, cudaStream_t st);
 
 }  // namespace mlxq

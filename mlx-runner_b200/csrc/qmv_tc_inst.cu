@@ -57,6 +57,33 @@ static cudaError_t launch_tokens(const MmaParams& p, const TcPlan& tp, size_t sm
     }
 }
 
+#if MLXQ_BITS == 4
+int qmv_tc_clusters(int kz, size_t smem) {
+    const auto kernel = qmv_tc_kernel<4, 8, 2>;
+    int dev = 0, sms = 0, n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute la[1];
+    la[0].id = cudaLaunchAttributeClusterDimension;
+    la[0].val.clusterDim.x = static_cast<unsigned>(kz);
+    la[0].val.clusterDim.y = la[0].val.clusterDim.z = 1;
+    cfg.blockDim = dim3(TC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = la;
+    cfg.numAttrs = 1;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_WHOLE) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    cfg.gridDim = dim3(static_cast<unsigned>(2 * sms / kz * kz));
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+#endif
+
 cudaError_t MLXQ_CAT(launch_qmv_tc_b, MLXQ_BITS)(const MmaParams& p, const TcPlan& tp, size_t smem, int device, cudaStream_t st) {
     return p.split == 2 ? launch_tokens<2>(p, tp, smem, device, st) : launch_tokens<1>(p, tp, smem, device, st);
 }

@@ -23,9 +23,9 @@ def plans(tmp_path_factory):
     objs = [os.path.join(build.OBJ, o) for (_, o, _) in build.UNITS]
     subprocess.run([build._nvcc()] + build.COMMON + ["-I", build.CSRC, os.path.join(HERE, "decode_plans.cu"), "-o", exe] + objs + ["-ldl"], check=True)
 
-    def run(calls):
+    def run(calls, *args):
         text = "\n".join(" ".join(str(v) for v in c) for c in calls)
-        out = subprocess.run([exe], input=text, capture_output=True, text=True, check=True).stdout.splitlines()
+        out = subprocess.run([exe, *args], input=text, capture_output=True, text=True, check=True).stdout.splitlines()
         assert len(out) == len(calls)
         return [[[int(v) for v in part.split()] for part in line.split("|")] for line in out]
 
@@ -46,7 +46,7 @@ def test_no_row_length_leaves_the_shared_memory_asked_for(plans):
              for bits, gs, rows, tokens, split in ((4, 64, 128, 16, 2), (8, 32, 40, 8, 2), (4, 128, 4096, 16, 1), (2, 64, 24, 3, 2), (6, 32, 64, 6, 2))]
     served = 0
     for call, (tc, *others) in zip(calls, plans(calls)):
-        smem, kz, stages, depth, off_x, off_xsum, off_red, off_bars = tc
+        smem, kz, stages, depth, off_x, off_xsum, off_red, off_bars, *_ = tc
         if smem:
             served += 1
             bits, gs, k, rows, tokens, split, _ = call
@@ -59,3 +59,15 @@ def test_no_row_length_leaves_the_shared_memory_asked_for(plans):
                 served += 1
                 assert plan[0] <= SMEM_OPT_IN and all(a <= b for a, b in zip([1] + plan[1:], plan[1:] + [plan[0]])), f"{call}: {plan}"
     assert served > 300
+
+
+def test_clusters_are_the_ones_that_the_device_holds(plans):
+    calls = [(4, 64, k, rows, tokens, 2, 1) for k in (1024, 4096, 12288) for rows in (128, 4096, 40960) for tokens in (2, 6, 16)]
+    for args, room in (((), {1: 296, 2: 148, 4: 71, 8: 33}), (("part",), {1: 40, 2: 20, 4: 10})):
+        cuts = set()
+        for call, (tc, *_) in zip(calls, plans(calls, *args)):
+            if tc[0]:
+                kz, clusters, n_blocks = tc[1], tc[-2], tc[-1]
+                assert kz in room and 1 <= clusters <= min(room[kz], n_blocks), f"{call}: {tc}"
+                cuts.add(kz)
+        assert cuts >= set(room) - {1, 2}, cuts
