@@ -58,8 +58,13 @@ static cudaError_t launch_tokens(const MmaParams& p, const TcPlan& tp, size_t sm
 }
 
 #if MLXQ_BITS == 4
+// (an empty kernel of the same block and shared memory: for one that allocates tensor memory the occupancy calls say one CTA an
+// SM whatever its shared memory, although two of these run side by side -- 24576 x 2048, 4 bits, 16 fp32 tokens, planned for one
+// CTA an SM 44.7 us, for two 24.6)
+static __global__ void __launch_bounds__(TC_THREADS, 2) qmv_tc_shape() {}
+
 int qmv_tc_clusters(int kz, size_t smem) {
-    const auto kernel = qmv_tc_kernel<4, 8, 2>;
+    const auto kernel = qmv_tc_shape;
     int dev = 0, sms = 0, n = 0;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute la[1];
