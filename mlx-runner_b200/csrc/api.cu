@@ -293,24 +293,26 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
             return MLXQ_OK;
         }
     }
+    // Small batches that the tensor-memory kernel is the faster one for, by what they run on otherwise: its status, or -1.
     // (A shard keeps to the kernels that can store into the peers' windows, so that its rows are the same bits whichever way they
     // are gathered.)
     bool sharded = false;
     for (int i = 0; i < n; i++) sharded = sharded || parts[i]->shard_count > 1;
-    if (T >= 2 && T <= 16 && !sharded && (mode == Decode::any || mode == Decode::tc)) {
-        // small batches: the tensor-memory kernel where it serves the call and is the faster one
+    const auto tensor_memory = [&](TcInstead instead) -> int {
+        if (T < 2 || T > 16 || sharded || (mode != Decode::any && mode != Decode::tc)) return -1;
         MmaParams mt = {};
         p.T = static_cast<int>(T); p.x = x; p.y = y;
         mt.q = p;
         mt.split = x_dtype == MLXQ_F32 ? 2 : 1;
         mt.err = device_error_word(parts[0]->device);
         TcPlan tc;
-        const size_t tsmem = mt.err ? qmv_tc_plan(parts[0]->bits, mt, static_cast<int>(T), mode == Decode::tc, qmv_tc_room(parts[0]->device, device_sm_count(parts[0]->device)), tc) : 0;
-        if (tsmem) {
-            const cudaError_t err = launch_qmv_tc(parts[0]->bits, mt, tc, tsmem, parts[0]->device, st);
-            return err == cudaSuccess ? MLXQ_OK : cuda_fail(err, "qmv (tensor memory) launch");
-        }
-    }
+        const size_t tsmem = mt.err ? qmv_tc_plan(parts[0]->bits, mt, static_cast<int>(T), instead, qmv_tc_room(parts[0]->device, device_sm_count(parts[0]->device)), tc) : 0;
+        if (!tsmem) return -1;
+        const cudaError_t err = launch_qmv_tc(parts[0]->bits, mt, tc, tsmem, parts[0]->device, st);
+        return err == cudaSuccess ? MLXQ_OK : cuda_fail(err, "qmv (tensor memory) launch");
+    };
+    if (mode == Decode::tc)
+        if (const int rc = tensor_memory(TcInstead::named); rc >= 0) return rc;
     MmaParams mp;
     bool planned = false;
     const size_t smem = mma_plan(parts, n, x_dtype, T, mp, &planned);
@@ -327,6 +329,7 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
             TokPlan tp;
             const size_t tsmem = qmv_tok_plan(parts[0]->bits, mp, static_cast<int>(T), device_sm_count(parts[0]->device), tp);
             if (tsmem) {
+                if (const int rc = tensor_memory(TcInstead::token_major); rc >= 0) return rc;
                 const cudaError_t err = launch_qmv_tok(parts[0]->bits, mp, tp, tsmem, parts[0]->device, st);
                 if (err != cudaSuccess) return cuda_fail(err, "qmv (token-major) launch");
                 return MLXQ_OK;
@@ -364,12 +367,14 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
             TokPlan tp;
             const size_t tsmem = qmv_tok_plan(bits, mp, static_cast<int>(T), device_sm_count(parts[0]->device), tp, fit == 4 ? 1 : 2);
             if (tsmem) {
+                if (const int rc = tensor_memory(fit == 4 ? TcInstead::cluster : TcInstead::scaled_cluster); rc >= 0) return rc;
                 const cudaError_t err = launch_qmv_tok(parts[0]->bits, mp, tp, tsmem, parts[0]->device, st);
                 if (err != cudaSuccess) return cuda_fail(err, "qmv (token-major, cluster) launch");
                 return MLXQ_OK;
             }
         }
         if (peer && !rsmem) return fail(MLXQ_UNSUPPORTED, "this shape does not run on the persistent decode kernel: no fused gather");
+        if (const int rc = tensor_memory(fit == 4 ? TcInstead::halves : TcInstead::other); rc >= 0) return rc;
         if (fit) {
             // ... or two calls of half the tokens: each on a persistent kernel, they beat the register-fed kernel although
             // the weights are read twice.
@@ -389,6 +394,8 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
     }
     if (peer) return fail(MLXQ_UNSUPPORTED, "this shape does not run on the persistent decode kernel: no fused gather");
     if (x_up) return fail(MLXQ_UNSUPPORTED, "this shape does not run on the persistent decode kernels: no gated input");
+    if (!planned)
+        if (const int rc = tensor_memory(TcInstead::other); rc >= 0) return rc;
     // gridDim.y carries token tiles of four; walk very long batches in slices.
     const int64_t slice = 4 * 65535;
     for (int64_t t0 = 0; t0 < T; t0 += slice) {

@@ -19,31 +19,77 @@ namespace {
 
 int align_up(int v, int a) { return (v + a - 1) / a * a; }
 
-// Whether the kernel is the faster one for a call that others could serve, and no less exact.  Both sides in us, this kernel's
-// first; 4 bits in groups of 64 unless it says otherwise.
-bool worth(int bits, int gs, int K, int rows, int tokens, int split) {
-    // 6 and 8 bits in groups of 128: long sums of uncentred codes, whose error is above the token-major kernel's (8 bits, fp32
-    // tokens 4.4e-7 of the result against 3.4e-7; in groups of 64 3.1e-7 against 3.7e-7)
-    if (bits >= 6 && gs == 128) return false;
-    // more fp32 tokens than the others take at once: 1024 x 1024, 16 tokens 5.7 : 8.3; 4096 x 4096 12.3 : 24.8; 4096 x 12288
-    // 37 : 231; 24576 x 4096 42 : 72; 11008 x 4096 at 3 bits 31 : 361
-    if (split == 2 && tokens > 8) return true;
-    // short rows: the fixed part of a launch decides (6 fp32 tokens: 4096 x 1024 at 8 bits 5.8 : 5.3, 1024 x 1024 4.5 : 4.1;
-    // 2048 x 2048 5.7 : 6.3, 1024 x 3072 at 8 bits 6.1 : 7.9)
-    if (K < 2048) return false;
-    // the token-major kernel's second eight columns.  6 fp32 tokens: 4096 x 4096 9.3 : 11.8, 4096 x 12288 15.5 : 24.4,
-    // 24576 x 4096 25.7 : 33.4, 151936 x 4096 at 6 bits 152 : 158, at 8 bits 140 : 153
-    if (split == 2 && tokens > 4) return true;
-    // 13 fp16 tokens (sixteen columns drained): 4096 x 4096 12.0 : 13.6, 4096 x 12288 23 : 36, 11008 x 4096 at 3 bits 25.6 : 31.0,
-    // but 24576 x 4096 36.8 : 36.8, 14336 x 4096 at 8 bits 27.2 : 26.0, 151936 x 4096 at 8 bits 197 : 164
-    if (split == 1 && tokens > 8) return rows <= (bits == 8 ? 8192 : 12288);
-    if (bits == 8) return false;                               // 14336 x 4096, 4 fp32 tokens 18.2 : 16.8, 8 fp16 ones 21.3 : 18.6
-    // 4 fp32 tokens: 4096 x 4096 8.6 : 9.2, 24576 x 4096 22.3 : 25.8, 40960 x 2048 19.6 : 22.1, 151936 x 4096 at 6 bits 145 : 130
-    if (split == 2 && tokens > 2) return rows <= 40960;
-    // 8 fp16 tokens: 4096 x 4096 9.8 : 10.4, 4096 x 12288 16.6 : 19.5, 24576 x 4096 26.6 : 27.6, 40960 x 2048 23.9 : 23.2
-    if (split == 1 && tokens > 4) return rows <= 24576;
-    // 2 fp32 tokens: 4096 x 12288 14.4 : 17.4, but 4096 x 4096 8.4 : 7.7
-    return split == 2 && tokens == 2 && K >= 8192 && rows <= 12288;
+// Whether the kernel is the faster one, by what the call runs on otherwise.  Fitted to 70,000 calls timed on both sides in turn: 6
+// widths, groups of 32, 64 and 128, 33 row counts of 512 ... 151936, 26 row lengths of 512 ... 14336, batches of 2 ... 16 tokens of
+// each type: of the 23,600 calls that the rules take, 0.6 % are more than 1.5 % slower than before, 7 by more than 10 %, and the mean is
+// 2.4 times as fast.  (11008 x 4096, 3 bits, 16 fp32 tokens, in the place of CUDA cores: 361 -> 32 us.)
+
+// In the place of one launch of the token-major kernel on single CTAs.  Each of its CTAs stages all of K of the batch: the KB of
+// that decide, less of them where few rows leave it few CTAs to a wave.  us before : with this
+// kernel, groups of 64: 6 fp32 tokens at 4 bits, 4096 x 4096 (96 KB) 12.1 : 10.1, 24576 x 4096 33.5 : 28.7, 24576 x 2048 17.7 : 17.9,
+// 4096 x 1024 5.8 : 6.8; 4 tokens 24576 x 4096 25.9 : 27.3; 6 tokens at 6 bits 151936 x 4096 159 : 175; 8 fp16 tokens at 3 bits
+// 11008 x 4096 (64 KB) 22.5 : 20.3.
+bool over_token_major(int bits, int gs, int rows, int tokens, int split, int kb) {
+    const bool even = bits == 4 || bits == 8, fp32 = split == 2;
+    if (gs == 32 && bits == 4 && !fp32) return false;
+    if (tokens <= 4) {
+        // (few tokens: the other kernel has one set of accumulators and few staged columns)
+        if (!fp32) return false;
+        if (tokens == 2) return gs == 64 && bits <= 5 && rows <= 6144 && kb >= 80 && kb <= 96;
+        if (rows <= 3072) return kb >= (gs == 128 && !even ? 40 : 80);
+        if (gs == 32) return bits >= 6 && kb >= (rows <= 15360 ? 72 : 48);
+        if (gs == 128 || bits >= 6) return false;
+        if (rows <= 15360) return kb >= 80 && (bits != 2 || rows <= 6144);
+        return bits != 2 && kb >= (bits == 4 ? 144 : 112);
+    }
+    if (gs == 32) return kb >= (rows <= 3072 || bits == 4 || !fp32 || (bits == 6 && rows <= 15360) ? 96 : 56);
+    if (gs == 128) {
+        if (!even) return rows <= 15360 && kb >= (rows <= 3072 ? 32 : rows <= 6144 ? 40 : 64);
+        if (rows <= 3072) return kb >= (bits == 4 ? 56 : 40);
+        return bits == 8 && fp32 && kb >= (rows <= 6144 ? 40 : 64);
+    }
+    if (rows <= 3072) return kb >= (fp32 || even ? 48 : rows <= 1536 ? 32 : 40);
+    if (rows <= 6144) return kb >= (bits == 8 ? 112 : bits == 4 ? 72 : fp32 ? 64 : 56);
+    if (fp32) {
+        if (rows <= 15360) return kb >= (bits >= 6 ? 112 : bits == 5 ? 80 : 72);
+        return bits >= 3 && bits <= 5 && kb >= (bits == 3 ? 96 : bits == 5 ? 80 : 72);
+    }
+    if (tokens <= 8 && bits >= 3 && bits <= 5) return kb >= (bits == 5 ? 72 : bits == 3 && rows <= 15360 ? 64 : 96);
+    return rows <= 15360 && !even && kb >= 112;
+}
+
+// ... of the token-major kernel with K split over a cluster, `scaled` or not: mostly the taller layers, where its clusters queue
+// (8 fp32 tokens, 4 bits, 11008 x 12288 60.9 : 41.0 us; 6 bits 61.4 : 64.2).
+bool over_cluster(int bits, int gs, int rows, int tokens, int split, bool scaled) {
+    const bool fp32 = split == 2;
+    if (tokens <= 4 || gs == 128) return false;
+    if (gs == 32) return fp32 && bits >= 6 && rows > 3072;
+    if (!scaled)
+        return fp32 && ((bits == 4 && rows > (tokens >= 6 ? 3072 : 6144)) || (bits == 5 && rows > 6144) || (bits == 3 && rows > 32768));
+    switch (bits) {
+        case 2: return rows <= (fp32 ? 15360 : 3072);
+        case 3: return rows > 6144 && (fp32 || rows <= 15360);
+        case 4: return fp32 || rows <= 15360;
+        case 5: return rows > 3072;
+        default: return false;
+    }
+}
+
+bool worth(TcInstead instead, int bits, int gs, int K, int rows, int tokens, int split) {
+    switch (instead) {
+        case TcInstead::named: return true;
+        case TcInstead::token_major: return over_token_major(bits, gs, rows, tokens, split, tokens * split * (K / 128) / 4);      // (K <= STAGED_K_MAX)
+        case TcInstead::cluster: return over_cluster(bits, gs, rows, tokens, split, false);
+        case TcInstead::scaled_cluster: return over_cluster(bits, gs, rows, tokens, split, true);
+        case TcInstead::halves:
+            // two launches of the token-major kernel, which read the weights twice.  Not where they are near the memory's rate all the
+            // same: vocabulary-sized layers, at 8 bits on rows that cut badly (100352 x 2560, 16 fp32 tokens 140 : 205 us), in groups of 128,
+            // and at 6 bits on very short rows
+            if (rows > 32768 && ((bits == 8 && K > 2048 && K < 4096) || (gs == 128 && K > 3072 && K < 8192))) return false;
+            if (rows > 20480 && bits == 6 && K < 1024) return false;
+            return true;
+        default: return tokens >= (split == 2 ? 3 : 5);        // kernels on the CUDA cores, or that read the weights several times
+    }
 }
 
 }  // namespace
@@ -65,11 +111,11 @@ const TcRoom& qmv_tc_room(int device, int sms) {
     return r;
 }
 
-size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, bool always, const TcRoom& room, TcPlan& tp) {
+size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, TcInstead instead, const TcRoom& room, TcPlan& tp) {
     const QmvParams& q = p.q;
     if (q.K > STAGED_K_MAX || tokens < 2 || tokens > 16 || q.peer.n > 0 || q.x_up != nullptr || q.e != nullptr) return 0;
     if ((q.gs != 32 && q.gs != 64 && q.gs != 128) || (q.s_dtype != DT_F16 && q.s_dtype != DT_BF16) || q.K % TC_STAGE != 0) return 0;
-    if (!always && !worth(bits, q.gs, q.K, q.total_rows, tokens, p.split)) return 0;
+    if (!worth(instead, bits, q.gs, q.K, q.total_rows, tokens, p.split)) return 0;
     tp = TcPlan{};
     uintptr_t at = 16;
     for (int i = 0; i < q.n_parts; i++) {
@@ -81,23 +127,28 @@ size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, bool always, const 
     }
     tp.s_align = static_cast<int>(at & (~at + 1));
     tp.stages = q.K / TC_STAGE;
-    // The cut of K: the one that is done first by what was measured (6 fp32 tokens, 4 bits): a stage takes 0.8 us where two CTAs
-    // share an SM and 0.47 where one has it, the end of a block and its slices' meeting 2 us.  24576 x 4096 in 2, 4 and 8
-    // slices: 30.1, 25.7, 31.9 us; 40960 x 2048: 22.3, 26.6, 37.8; 4096 x 4096: 13.9, 10.5, 9.3.  (From the tokens the kernel
-    // is compiled for, not the batch's: a token's sums do not change with its company.)
+    // The cut of K: the one that is done first by a cost in units of a stage of 128 codes on a CTA that has its SM alone.  Fitted
+    // to the times of all four cuts at 6 widths, 14 row counts, 8 row lengths and 11 batches: the cut it takes is 1.1 % slower
+    // than the best one on average, and 4 % at the ninth decile.  What it says: two CTAs an SM hide nearly all of a stage, so that
+    // little but the staging of the activations (per stage, token and part; four times the stores at the widths whose codes
+    // straddle bytes) and the blocks' ends are left to count.  11008 x 4096, 3 bits, 8 fp16 tokens in 2 and 8 slices: 34.2 and
+    // 20.3 us; 24576 x 4096, 4 bits, 16 fp32 tokens in 2 and 8 slices: 55.2 and 45.1.  (From the tokens the kernel is compiled for,
+    // not the batch's: a token's sums do not change with its company.)
     const int ntk = tc_tokens(tokens), part = ntk <= 8 ? 1024 : 2048, slot = tc_slot_bytes(bits);
-    // 16-bit activations at 8 bits, and at 5 and 6 bits in groups of 32: the call stands in for kernels that multiply and add in
-    // fp32, whose error grows with the number of groups and codes that one CTA sums up.  Error of the result, this kernel's first
-    // (16 bf16 tokens): 8 bits in groups of 32, 48 groups of 12288 codes 1.42e-7 : 1.19e-7 and 28 groups of 8192 codes below
-    // theirs; in groups of 64, 3072 codes 1.39e-7 : 1.19e-7, 1792 codes 1.19e-7 : 1.24e-7.
-    const bool fp32_stand_in = p.split == 1 && (bits == 8 || (bits >= 5 && q.gs == 32));
+    // 16-bit activations at 8 bits, and at 6 bits in groups of 32: the call stands in for kernels that multiply and add in fp32, and
+    // the error here grows with the groups and codes that one CTA sums up.  Error of the result, this kernel's first (16 bf16
+    // tokens): 8 bits in groups of 32, 48 groups of 12288 codes 1.42e-7 : 1.19e-7, 32 groups of 8192 codes below theirs; in groups
+    // of 64, 3072 codes 1.39e-7 : 1.19e-7, 1792 codes 1.19e-7 : 1.24e-7; 6 bits, 96 groups 1.85e-7 : 1.73e-7, 48 groups
+    // 1.41e-7 : 1.65e-7.
+    const bool fp32_stand_in = p.split == 1 && (bits == 8 || (bits == 6 && q.gs == 32));
+    const int most_codes = bits == 8 ? 2048 : 1536, most_groups = bits == 8 ? 32 : 48;
     double best = 0.0;
     size_t best_smem = 0;
     for (int shift = 0; shift <= 3; shift++) {
         const int kz = 1 << shift;
         if (kz > tp.stages) continue;
         const int slice = (tp.stages + kz - 1) / kz;
-        if (fp32_stand_in && (slice * TC_STAGE > 2048 || slice * TC_STAGE / q.gs > 32)) continue;
+        if (fp32_stand_in && (slice * TC_STAGE > most_codes || slice * TC_STAGE / q.gs > most_groups)) continue;
         const int x_bytes = slice * 2 * p.split * part, xsum = align_up((slice * TC_STAGE / q.gs) * ntk * 8, 16), redb = 2 * ntk * 128 * 4;
         const int fixed = 1024 + x_bytes + xsum + redb + static_cast<int>(sizeof(TcBarriers));
         const bool two = fixed + 3 * slot <= TC_SMEM_TWO;
@@ -107,7 +158,8 @@ size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, bool always, const 
         const int resident = (two ? room.two : room.one)[shift], clusters = tp.n_blocks < resident ? tp.n_blocks : resident;
         if (clusters < 1) continue;
         const int rounds = (tp.n_blocks + clusters - 1) / clusters;
-        const double cost = rounds * (slice * (clusters * kz > room.sms ? 0.8 : 0.47) + 2.0);
+        const double staging = (bits == 3 || bits == 5 || bits == 6 ? 0.04 : 0.025) * ntk * (p.split + 1);
+        const double cost = slice * staging + rounds * (slice * (clusters * kz > room.sms ? 0.07 : 1.0) + 0.25 + 0.3 * shift);
         if (best_smem != 0 && cost >= best) continue;
         best = cost;
         tp.kz = kz; tp.kz_shift = shift; tp.clusters = clusters; tp.depth = depth;

@@ -629,9 +629,12 @@ struct TcRoom {
 };
 const TcRoom& qmv_tc_room(int device, int sms);
 
-// Plans a call; returns the shared memory it needs, 0 when the call is not one the kernel serves or, unless `always`, not one
-// that it is the faster for.
-size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, bool always, const TcRoom& room, TcPlan& tp);
+// What a call runs on where the kernel does not take it: `named` is a call that the kernel takes whenever it can serve it.
+enum class TcInstead { named, token_major, cluster, scaled_cluster, halves, other };
+
+// Plans a call; returns the shared memory it needs, 0 when the call is not one the kernel serves, or not one that it is the faster
+// for than what the call runs on otherwise.
+size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, TcInstead instead, const TcRoom& room, TcPlan& tp);
 cudaError_t launch_qmv_tc(int bits, const MmaParams& p, const TcPlan& tp, size_t smem, int device, cudaStream_t st);
 
 }  // namespace mlxq

@@ -11,8 +11,8 @@ using namespace mlxq;
 int main(int argc, char** argv) {
     TcRoom room = {148, {148, 74, 33, 15}, {296, 148, 71, 33}};         // a B200
     if (argc > 1) room = TcRoom{20, {20, 10, 5, 0}, {40, 20, 10, 0}};   // a part of one that holds no cluster of eight
-    int bits, gs, K, rows, tokens, split, always;
-    while (std::scanf("%d %d %d %d %d %d %d", &bits, &gs, &K, &rows, &tokens, &split, &always) == 7) {
+    int bits, gs, K, rows, tokens, split, instead;
+    while (std::scanf("%d %d %d %d %d %d %d", &bits, &gs, &K, &rows, &tokens, &split, &instead) == 7) {
         MmaParams p = {};
         QmvParams& q = p.q;
         for (QmvPart& part : q.part) {
@@ -30,7 +30,7 @@ int main(int argc, char** argv) {
         for (int s = 3; s < 31; s++) if ((1 << s) == gs) q.gs_shift = s;
         p.split = split;
         TcPlan tc = {};
-        const size_t tcs = qmv_tc_plan(bits, p, tokens, always != 0, room, tc);
+        const size_t tcs = qmv_tc_plan(bits, p, tokens, static_cast<TcInstead>(instead), room, tc);
         std::printf("%zu %d %d %d %d %d %d %d %d %d", tcs, tc.kz, tc.stages, tc.depth, tc.off_x, tc.off_xsum, tc.off_red, tc.off_bars, tc.clusters, tc.n_blocks);
         const bool columns = qmv_mma_plan(bits, K, gs, tokens * split, p);
         for (int clusters = 0; clusters <= 2; clusters++) {

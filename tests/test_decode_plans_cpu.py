@@ -10,6 +10,7 @@ ROOT = os.path.dirname(HERE)
 PKG = os.path.join(ROOT, "mlx-runner_b200")
 
 SMEM_OPT_IN = 227 * 1024
+NAMED, TOKEN_MAJOR, CLUSTER, SCALED_CLUSTER, HALVES, OTHER = range(6)       # enum TcInstead
 
 
 @pytest.fixture(scope="module")
@@ -42,7 +43,7 @@ def test_no_row_length_leaves_the_shared_memory_asked_for(plans):
             lengths.update(at + d * 128 for d in (-80, -3, -1, 0, 1, 2, 40) if 1024 <= at + d * 128 <= 1 << 30)
     lengths.update(range(1024, 1 << 18, 640))
     lengths.update(range(1 << 18, 1 << 30, 1021 * 1024))
-    calls = [(bits, gs, k // 128 * 128, rows, tokens, split, 1) for k in sorted(lengths)
+    calls = [(bits, gs, k // 128 * 128, rows, tokens, split, NAMED) for k in sorted(lengths)
              for bits, gs, rows, tokens, split in ((4, 64, 128, 16, 2), (8, 32, 40, 8, 2), (4, 128, 4096, 16, 1), (2, 64, 24, 3, 2), (6, 32, 64, 6, 2))]
     served = 0
     for call, (tc, *others) in zip(calls, plans(calls)):
@@ -62,7 +63,7 @@ def test_no_row_length_leaves_the_shared_memory_asked_for(plans):
 
 
 def test_clusters_are_the_ones_that_the_device_holds(plans):
-    calls = [(4, 64, k, rows, tokens, 2, 1) for k in (1024, 4096, 12288) for rows in (128, 4096, 40960) for tokens in (2, 6, 16)]
+    calls = [(4, 64, k, rows, tokens, 2, NAMED) for k in (1024, 4096, 12288) for rows in (128, 4096, 40960) for tokens in (2, 6, 16)]
     for args, room in (((), {1: 296, 2: 148, 4: 71, 8: 33}), (("part",), {1: 40, 2: 20, 4: 10})):
         cuts = set()
         for call, (tc, *_) in zip(calls, plans(calls, *args)):
@@ -71,3 +72,26 @@ def test_clusters_are_the_ones_that_the_device_holds(plans):
                 assert kz in room and 1 <= clusters <= min(room[kz], n_blocks), f"{call}: {tc}"
                 cuts.add(kz)
         assert cuts >= set(room) - {1, 2}, cuts
+
+
+# (bits, group, K, rows, tokens, fp16 parts per activation), what the call runs on otherwise, and whether the tensor-memory kernel takes it
+@pytest.mark.parametrize("call,instead,taken", [
+    # 3 bits, 8 fp16 tokens of 4096 codes (64 KB staged by a CTA of the token-major kernel): the tallest layers stay there
+    ((3, 64, 4096, 11008, 8, 1), TOKEN_MAJOR, True), ((3, 64, 4096, 15368, 8, 1), TOKEN_MAJOR, False), ((2, 128, 4096, 16384, 8, 1), TOKEN_MAJOR, False),
+    # the batch of six of a 4-bit decode step, its 6-bit vocabulary head, and its neighbours in tokens
+    ((4, 64, 4096, 24576, 6, 2), TOKEN_MAJOR, True), ((4, 64, 4096, 4096, 6, 2), TOKEN_MAJOR, True), ((4, 64, 12288, 4096, 6, 2), CLUSTER, True),
+    ((6, 64, 4096, 151936, 6, 2), TOKEN_MAJOR, False), ((4, 64, 4096, 24576, 4, 2), TOKEN_MAJOR, False), ((4, 64, 2048, 24576, 6, 2), TOKEN_MAJOR, False),
+    # on either side of the rows that a limit stands at
+    ((5, 64, 4096, 3072, 5, 1), TOKEN_MAJOR, True), ((5, 64, 4096, 3080, 5, 1), TOKEN_MAJOR, False),
+    ((8, 64, 4096, 3072, 6, 2), TOKEN_MAJOR, True), ((8, 64, 4096, 3080, 6, 2), TOKEN_MAJOR, False),
+    # two launches of half the tokens; not vocabulary-sized layers at 8 bits on rows that cut badly
+    ((8, 64, 2560, 32768, 16, 2), HALVES, True), ((8, 64, 2560, 32776, 16, 2), HALVES, False), ((4, 64, 2560, 151936, 16, 2), HALVES, True),
+    # in the place of kernels without tensor cores, from three fp32 or five 16-bit tokens on
+    ((2, 32, 512, 4096, 3, 2), OTHER, True), ((2, 32, 512, 4096, 2, 2), OTHER, False), ((2, 32, 512, 4096, 5, 1), OTHER, True), ((2, 32, 512, 4096, 4, 1), OTHER, False),
+    # 8 bits with 16-bit activations: while the sums are short enough
+    ((8, 32, 8192, 4096, 16, 1), OTHER, True), ((8, 32, 12288, 4096, 16, 1), OTHER, False), ((8, 64, 14336, 4096, 16, 1), OTHER, True),
+    # what the kernel cannot serve
+    ((4, 64, 4096 + 64, 4096, 6, 2), NAMED, False), ((4, 64, 4096, 4096, 17, 2), NAMED, False), ((4, 64, 4096, 4096, 1, 2), NAMED, False),
+])
+def test_which_small_batches_the_tensor_memory_kernel_takes(plans, call, instead, taken):
+    assert (plans([call + (instead,)])[0][0][0] > 0) == taken
