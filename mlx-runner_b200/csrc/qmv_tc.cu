@@ -115,7 +115,7 @@ size_t qmv_tc_plan(int bits, const MmaParams& p, int tokens, TcInstead instead, 
     const QmvParams& q = p.q;
     if (q.K > STAGED_K_MAX || tokens < 2 || tokens > 16 || q.peer.n > 0 || q.x_up != nullptr || q.e != nullptr) return 0;
     if ((q.gs != 32 && q.gs != 64 && q.gs != 128) || (q.s_dtype != DT_F16 && q.s_dtype != DT_BF16) || q.K % TC_STAGE != 0) return 0;
-    if (!worth(instead, bits, q.gs, q.K, q.total_rows, tokens, p.split)) return 0;
+    if (!tc_compiled(bits, tc_tokens(tokens), p.split) || !worth(instead, bits, q.gs, q.K, q.total_rows, tokens, p.split)) return 0;
     tp = TcPlan{};
     uintptr_t at = 16;
     for (int i = 0; i < q.n_parts; i++) {

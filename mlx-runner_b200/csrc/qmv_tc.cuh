@@ -54,6 +54,9 @@ static_assert(TC_SD * TC_D_COLS + TC_SA * TC_A_COLS <= TC_TMEM, "tensor memory")
 // the batch (of two tokens or more) rounded up to the tokens a kernel is compiled for
 __host__ __device__ constexpr int tc_tokens(int t) { return t <= 2 ? 2 : t <= 4 ? 4 : t <= 8 ? 8 : 16; }
 
+// ... and whether it is compiled: 16-bit activations take the kernel from five tokens on, two fp32 tokens up to five bits
+__host__ __device__ constexpr bool tc_compiled(int bits, int ntk, int split) { return split == 1 ? ntk >= 8 : ntk > 2 || bits <= 5; }
+
 struct TcBarriers {
     uint64_t full_a[TC_SA], empty_a[TC_SA];
     uint64_t d_full[TC_SD], d_empty[TC_SD];

@@ -15,36 +15,40 @@ namespace mlxq {
 
 template <int NTK, int SPLIT>
 static cudaError_t launch_one(const MmaParams& p, const TcPlan& tp, size_t smem, int device, cudaStream_t st) {
-    // the shared-memory opt-in is an attribute of the function in one device's context
-    static std::mutex mu;
-    static bool done[64] = {};
-    if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!done[device]) {
-            const cudaError_t e = cudaFuncSetAttribute(qmv_tc_kernel<MLXQ_BITS, NTK, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_WHOLE);
-            if (e != cudaSuccess) return e;
-            done[device] = true;
+    if constexpr (!tc_compiled(MLXQ_BITS, NTK, SPLIT)) {
+        return cudaErrorNotSupported;
+    } else {
+        // the shared-memory opt-in is an attribute of the function in one device's context
+        static std::mutex mu;
+        static bool done[64] = {};
+        if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            if (!done[device]) {
+                const cudaError_t e = cudaFuncSetAttribute(qmv_tc_kernel<MLXQ_BITS, NTK, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_WHOLE);
+                if (e != cudaSuccess) return e;
+                done[device] = true;
+            }
         }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(tp.clusters * tp.kz));
+        cfg.blockDim = dim3(TC_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute la[2];
+        la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        la[0].val.programmaticStreamSerializationAllowed = 1;
+        int n = pdl_enabled() ? 1 : 0;
+        if (tp.kz > 1) {
+            la[n].id = cudaLaunchAttributeClusterDimension;
+            la[n].val.clusterDim.x = static_cast<unsigned>(tp.kz);
+            la[n].val.clusterDim.y = la[n].val.clusterDim.z = 1;
+            n++;
+        }
+        cfg.attrs = la;
+        cfg.numAttrs = static_cast<unsigned>(n);
+        return cudaLaunchKernelEx(&cfg, qmv_tc_kernel<MLXQ_BITS, NTK, SPLIT>, p, tp);
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(tp.clusters * tp.kz));
-    cfg.blockDim = dim3(TC_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute la[2];
-    la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    la[0].val.programmaticStreamSerializationAllowed = 1;
-    int n = pdl_enabled() ? 1 : 0;
-    if (tp.kz > 1) {
-        la[n].id = cudaLaunchAttributeClusterDimension;
-        la[n].val.clusterDim.x = static_cast<unsigned>(tp.kz);
-        la[n].val.clusterDim.y = la[n].val.clusterDim.z = 1;
-        n++;
-    }
-    cfg.attrs = la;
-    cfg.numAttrs = static_cast<unsigned>(n);
-    return cudaLaunchKernelEx(&cfg, qmv_tc_kernel<MLXQ_BITS, NTK, SPLIT>, p, tp);
 }
 
 template <int SPLIT>

@@ -95,3 +95,16 @@ def test_clusters_are_the_ones_that_the_device_holds(plans):
 ])
 def test_which_small_batches_the_tensor_memory_kernel_takes(plans, call, instead, taken):
     assert (plans([call + (instead,)])[0][0][0] > 0) == taken
+
+
+def test_every_compiled_kernel_is_one_that_the_dispatch_takes(plans):
+    # (width, tokens compiled for, parts): two fp32 tokens at 6 and 8 bits and four 16-bit ones and fewer are not compiled, not even
+    # where the kernel is named; every other instance is reached by some call
+    calls = [(bits, gs, k, rows, tokens, split, instead) for bits in (2, 3, 4, 5, 6, 8) for gs in (32, 64) for k in (2048, 4096, 8192, 11008, 12288)
+             for rows in (1024, 4096) for tokens in (2, 3, 4, 5, 8, 9, 16) for split in (1, 2) for instead in (NAMED, TOKEN_MAJOR, OTHER)]
+    named, chosen = set(), set()
+    for (bits, _, _, _, tokens, split, instead), (tc, *_) in zip(calls, plans(calls)):
+        if tc[0]:
+            (named if instead == NAMED else chosen).add((bits, 2 if tokens <= 2 else 4 if tokens <= 4 else 8 if tokens <= 8 else 16, split))
+    assert named == chosen
+    assert len(named) == 34 and not any(split == 1 and ntk <= 4 for _, ntk, split in named)
