@@ -56,3 +56,26 @@ def run(layer, x: np.ndarray, T: int, x_dtype=0, y_dtype=0, x_stride=None, y_str
     if ys > O:
         assert torch.isnan(yb[:, O:].float()).all(), "the kernel wrote into y's row padding"
     return out
+
+
+# Calls that take the tensor-memory kernel through its edges: (width, group, K, rows of the parts, tokens, activation type,
+# elements that the scales and biases start behind a 16-byte boundary, row bias).  test_decode_plans_cpu.py says what they reach.
+TENSOR_MEMORY_CALLS = [
+    (4, 64, 256, (128 * 296 * 6 + 72,), 5, 1, 0, False),        # one CTA a block, seven rounds of blocks
+    (4, 64, 1536, (128 * 148 * 5 + 8,), 8, 0, 0, False),        # two CTAs a block, six rounds
+    (3, 64, 1024, (128 * 71 * 5 + 40,), 16, 0, 0, False),       # four, six rounds
+    (8, 32, 4096, (128 * 33 * 5 + 120,), 12, 0, 0, False),      # eight, six rounds
+    (2, 64, 1152, (136, 392, 1000), 6, 0, 0, True),             # three parts that end inside a block, row bias, nine stages in eight slices
+    (5, 64, 4096, (8, 2056, 24), 13, 2, 0, True),
+    (6, 128, 640, (200,), 9, 0, 0, False),                      # five groups
+    (4, 128, 2176, (1000, 72), 16, 1, 0, False),                # seventeen
+    (4, 128, 128, (17,), 8, 0, 0, False),                       # one stage, one group
+    (8, 128, 384, (129,), 3, 0, 1, False),                      # scales on two bytes only
+    (4, 64, 4096, (1000,), 4, 0, 2, True),                      # on four
+    (2, 32, 4096, (4096,), 16, 1, 1, False),
+    (8, 64, 14336, (2056,), 16, 0, 0, False),                   # one CTA an SM, a short ring
+    (4, 64, 14336, (264,), 2, 0, 0, False),
+    (3, 32, 4096, (4000,), 7, 0, 0, False),
+    (6, 64, 2048, (5000,), 8, 2, 0, False),
+    (5, 32, 512, (31 * 128 + 1,), 4, 0, 4, False),
+]

@@ -5,6 +5,8 @@ import subprocess
 
 import pytest
 
+from helpers import TENSOR_MEMORY_CALLS
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 PKG = os.path.join(ROOT, "mlx-runner_b200")
@@ -108,3 +110,17 @@ def test_every_compiled_kernel_is_one_that_the_dispatch_takes(plans):
             (named if instead == NAMED else chosen).add((bits, 2 if tokens <= 2 else 4 if tokens <= 4 else 8 if tokens <= 8 else 16, split))
     assert named == chosen
     assert len(named) == 34 and not any(split == 1 and ntk <= 4 for _, ntk, split in named)
+
+
+def test_the_edges_that_the_gpu_tests_reach(plans):
+    # every cut with six rounds of blocks and more in at least one CTA (the sums' buffers are used again from the third on), every
+    # depth of the ring, an odd number of groups in a slice, fewer stages than turns that only fetch, all compiled batches
+    reached = [plans([(bits, gs, k, sum(rows), tokens, 2 if x_dtype == 0 else 1, NAMED)])[0][0]
+               for bits, gs, k, rows, tokens, x_dtype, _, _ in TENSOR_MEMORY_CALLS]
+    assert all(tc[0] for tc in reached)
+    assert {tc[1] for tc in reached if tc[-1] > 5 * tc[-2]} == {1, 2, 4, 8}
+    assert {tc[3] for tc in reached} == {3, 4, 6, 8}
+    assert any(tc[0] > 113 * 1024 for tc in reached)
+    assert any(k // gs % 2 for _, gs, k, *_ in TENSOR_MEMORY_CALLS) and min(tc[2] // tc[1] for tc in reached) == 1
+    assert {(2 if t <= 2 else 4 if t <= 4 else 8 if t <= 8 else 16, 2 if x == 0 else 1) for *_, t, x, _, _ in TENSOR_MEMORY_CALLS} == \
+        {(2, 2), (4, 2), (8, 2), (16, 2), (8, 1), (16, 1)}

@@ -20,6 +20,14 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-3
 
 
+def on_kernel(monkeypatch, name):
+    """MLXQ_DECODE (read at every call): the small-batch kernel to take, or the dispatch's own choice."""
+    if name is None:
+        monkeypatch.delenv("MLXQ_DECODE", raising=False)
+    else:
+        monkeypatch.setenv("MLXQ_DECODE", name)
+
+
 def close(oracle, got, ref, label, tol=TOL):
     err = oracle.max_rel_err(got, ref)
     assert err < tol, f"{label}: max relative error {err}"
@@ -160,12 +168,14 @@ def test_small_batch_fused_with_bias_matches_separate(mlxq, oracle):
         close(oracle, yd.cpu().numpy(), ref, f"fused q/k/v T {T}")
 
 
+@pytest.mark.parametrize("kernel", [None, "tok", "tc"])
 @pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
-def test_small_batches_every_width_and_group(mlxq, oracle, bits):
-    # Two to sixteen tokens take the decode kernel whose accumulator columns are tokens (where it serves the width and
-    # group size; the others fall to the general kernels): both 16-bit scale types, fp16 and fp32 activations, a row
+def test_small_batches_every_width_and_group(mlxq, oracle, monkeypatch, bits, kernel):
+    # Two to sixteen tokens take one of the two decode kernels whose accumulator columns are tokens (where they serve the width
+    # and group size; the others fall to the general kernels): both 16-bit scale types, fp16 and fp32 activations, a row
     # count that ends inside a block, group counts that leave windows of eight groups partly empty.  The bar is the
     # fp32 reassociation noise of a K-long sum, far below the 1e-3 of the reference's own tests.
+    on_kernel(monkeypatch, kernel)
     K, O = 1536, 72
     for gs in (32, 64, 128):
         for st in (oracle.F16, oracle.BF16):
@@ -179,11 +189,13 @@ def test_small_batches_every_width_and_group(mlxq, oracle, bits):
                 close(oracle, got, fx.reference(xr), f"bits {bits} gs {gs} st {st} T {T} x {x_dtype}", 1e-4 if x_dtype == 0 else 3e-5)
 
 
+@pytest.mark.parametrize("kernel", ["tok", "tc"])
 @pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
-def test_small_batches_of_long_rows(mlxq, oracle, bits):
+def test_small_batches_of_long_rows(mlxq, oracle, monkeypatch, bits, kernel):
     # rows of 6144 codes and more: single CTAs, and clusters where those do not hold the tokens -- even and uneven slices, fewer
     # blocks than clusters and several rounds of them, 16 tokens of 16-bit activations (a wider cluster where the slices do not
     # fit)
+    on_kernel(monkeypatch, kernel)
     for gs, K, O, T, x_dtype in ((64, 6144, 41, 2, 0), (32, 6656, 600, 6, 0), (128, 12288, 24, 8, 0), (64, 14336, 40, 16, 1), (64, 6400, 700, 5, 2),
                                 (64, 6144, 700, 8, 0), (64, 12288, 600, 6, 0), (64, 6144, 41, 16, 1), (128, 14336, 600, 10, 2)):
         fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=gs, scale_type=oracle.BF16, with_bias=(gs == 64), seed=bits + K)
@@ -198,10 +210,11 @@ def test_small_batches_of_long_rows(mlxq, oracle, bits):
 
 
 @pytest.mark.parametrize("T,O", [(5, 17), (5, 16 * 37 * 3), (7, 16 * 75), (5, 40)])
-def test_cluster_kernel_with_half_warps_at_different_turns(mlxq, oracle, T, O):
+def test_cluster_kernel_with_half_warps_at_different_turns(mlxq, oracle, monkeypatch, T, O):
     # odd tokens times odd blocks a cluster: the last rounds of the loops before the cluster's barriers, and of the block
     # ends, are run by half a warp.  One call after the other on the same buffers, so that a CTA that left early would
     # read the next call's sums.
+    on_kernel(monkeypatch, "tok")
     K, gs = 12288, 64
     fx = oracle.QuantFixture(O=O, K=K, bits=4, gs=gs, scale_type=oracle.BF16, seed=O)
     layer = DevLayer.from_fixture(mlxq, fx)
@@ -218,14 +231,16 @@ def test_cluster_kernel_with_half_warps_at_different_turns(mlxq, oracle, T, O):
 
 @pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
 @pytest.mark.parametrize("x_dtype,T", [(0, 7), (0, 8), (1, 12), (2, 13)])
-def test_cluster_kernel_at_any_magnitude(mlxq, oracle, bits, x_dtype, T):
-    # batches that the clusters serve in the place of kernels that multiply in fp32: tokens of 1e-30 ... 1e30 side by side, one
+@pytest.mark.parametrize("kernel", ["tok", "tc"])
+def test_cluster_kernel_at_any_magnitude(mlxq, oracle, monkeypatch, bits, x_dtype, T, kernel):
+    # batches that the clusters (and the tensor-memory kernel) serve in the place of kernels that multiply in fp32: tokens of 1e-30 ... 1e30 side by side, one
     # of zeros, one whose elements span ten orders of magnitude; in fp16 down to its subnormal numbers.  A token's power of two
     # leaves what lies above 2^-40 of its largest element as exact as at magnitude one; the bar there is that of the sums: the
     # uncentred codes' are up to four times the result's at 2 bits, 14336 terms in 16 slices, 2^-24 * sqrt(14336 / 16 / 8) * 4
     # and the bias term's as much again: 5e-6.
     if bits == 8 and x_dtype != 0:
         T = 8                                                      # (8 bits, 16-bit activations: two half batches, no cluster beyond)
+    on_kernel(monkeypatch, kernel)
     K, gs = 14336, 64
     for O in (40, 16 * 37 + 1):
         fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=gs, scale_type=oracle.BF16, seed=bits + O)
@@ -255,11 +270,14 @@ def test_cluster_kernel_at_any_magnitude(mlxq, oracle, bits, x_dtype, T):
 
 
 @pytest.mark.parametrize("x_dtype,T", [(0, 9), (0, 16), (2, 16), (0, 24), (2, 24)])
-def test_batches_beyond_the_persistent_kernels_keep_fp32_products(mlxq, oracle, x_dtype, T):
-    # calls that no persistent kernel holds on single CTAs, as one call or as two halves, multiply in fp32: activations of
-    # 1e5, which an fp16 operand cannot hold, and of 1e-5, which it holds to a few bits.  24 tokens: the paths without
+@pytest.mark.parametrize("kernel", [None, "tok"])
+def test_batches_beyond_the_persistent_kernels_keep_fp32_products(mlxq, oracle, monkeypatch, x_dtype, T, kernel):
+    # calls that no persistent kernel holds on single CTAs, as one call or as two halves, multiply in fp32, or on the
+    # tensor-memory kernel in scaled fp16 parts: activations of 1e5, which an fp16 operand cannot hold unscaled, and of 1e-5,
+    # which it holds to a few bits.  24 tokens: the paths without
     # scratch memory (static, captured, three layers in one launch).  The bar: fp32 sums of 14336 terms in 32 lanes, each
     # rounding 448 times (2^-24 * sqrt(448 / 3) = 7e-7 of the result; measured 3e-7).
+    on_kernel(monkeypatch, kernel)
     K, O, bits, gs = 14336, 24, 8, 64
     fx = oracle.QuantFixture(O=O, K=K, bits=bits, gs=gs, scale_type=oracle.BF16, seed=T)
     layer = DevLayer.from_fixture(mlxq, fx)

@@ -3,7 +3,7 @@ which of them takes a call, and the tensor-memory kernel at its edges, against t
 import pytest
 import torch
 
-from helpers import TORCH_DT, DevLayer, as_dtype
+from helpers import TENSOR_MEMORY_CALLS, TORCH_DT, DevLayer, as_dtype
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +92,70 @@ def test_no_less_exact_than_the_kernels_before(mlxq, monkeypatch, bits, gs, K, O
         torch.cuda.synchronize()
         err[mode] = ((y.double() - ref).norm() / ref.norm()).item()
     assert err[None] <= 1.05 * err["tok"], err
+
+
+@pytest.mark.parametrize("call", TENSOR_MEMORY_CALLS, ids=str)
+def test_tensor_memory_kernel_at_its_edges(mlxq, monkeypatch, call):
+    # against the same sums in 64 bits; x and y with padding, which must be neither read nor written
+    bits, gs, K, rows, T, x_dtype, offset, with_bias = call
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(K + T + bits)
+
+    def behind(t):
+        flat = torch.zeros(t.numel() + offset, dtype=t.dtype, device="cuda")
+        flat[offset:] = t.reshape(-1)
+        return flat[offset:].view(t.shape)
+
+    lins, refs, keep = [], [], []
+    x = torch.full((T, K + 8), float("nan"), device="cuda", dtype=TORCH_DT[x_dtype])
+    x[:, :K] = torch.randn((T, K), device="cuda", generator=gen).to(TORCH_DT[x_dtype])
+    for o in rows:
+        w = torch.randint(-(1 << 31), (1 << 31) - 1, (o, K * bits // 32), dtype=torch.int32, device="cuda", generator=gen)
+        s = (torch.randn((o, K // gs), device="cuda", generator=gen).abs() * 0.002 + 1e-4).to(torch.float16 if bits % 2 else torch.bfloat16)
+        b = (-float(1 << (bits - 1)) * s.float()).to(s.dtype)
+        bias = torch.randn(o, device="cuda", generator=gen).to(s.dtype) if with_bias else None
+        keep.append((w, behind(s), behind(b), bias))
+        lins.append(mlxq.Linear(*keep[-1], inDim=K))
+        wd = codes_of(w, bits, K).double() * s.double().repeat_interleave(gs, 1) + b.double().repeat_interleave(gs, 1)
+        refs.append(x[:, :K].double() @ wd.T + (bias.double() if with_bias else 0.0))
+    O = sum(rows)
+    ref = torch.cat(refs, 1)
+    y = torch.full((T, O + 3), float("nan"), device="cuda")
+    monkeypatch.setenv("MLXQ_DECODE", "tc")
+    for _ in range(2):
+        if len(lins) == 1:
+            lins[0].encode(None, x, K + 8, y, O + 3, T)
+        else:
+            mlxq.Linear.encodeFusedDecode(None, lins, x, y, K + 8, O + 3, T)
+    torch.cuda.synchronize()
+    mlxq.streamStatus(None, 0)
+    assert torch.isnan(y[:, O:]).all()
+    # a rounding of 2^-24 for each of the K / gs groups added up, of a running sum that holds up to the result's magnitude and, per
+    # group, of products some times larger; an fp32 activation's two parts leave 2^-22 of a product
+    bar = 2.0 ** -24 * (2.0 * (K / gs) ** 0.5 + 2.0)
+    err = ((y[:, :O].double() - ref).norm() / ref.norm()).item()
+    assert err < bar, f"{err} of the result, bar {bar}"
+    # no single output further off than such a sum can be: six deviations
+    worst = ((y[:, :O].double() - ref).abs().max() / ref.pow(2).mean().sqrt()).item()
+    assert worst < 6 * bar, f"{worst} of the root mean square"
+
+
+@pytest.mark.parametrize("bits,K,O,T,x_dtype", [(4, 4096, 24576, 6, 0), (4, 4096, 24576, 16, 1), (3, 4096, 11008, 16, 0), (8, 12288, 4096, 8, 0)])
+def test_tensor_memory_kernel_repeats_bit_for_bit_at_full_size(mlxq, monkeypatch, bits, K, O, T, x_dtype):
+    # sums are formed in a fixed order, and every wait before a tensor-memory store is by one polling lane: twelve calls of full
+    # size, one right after the other and with dependent launches in flight, give the same bits
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(O + T)
+    w = torch.randint(-(1 << 31), (1 << 31) - 1, (O, K * bits // 32), dtype=torch.int32, device="cuda", generator=gen)
+    s = (torch.rand((O, K // 64), device="cuda", generator=gen) * 0.004).to(torch.bfloat16)
+    lin = mlxq.Linear(w, s, (-float(1 << (bits - 1)) * s.float()).to(torch.bfloat16), None, inDim=K)
+    x = torch.randn((T, K), device="cuda", generator=gen).to(TORCH_DT[x_dtype])
+    monkeypatch.setenv("MLXQ_DECODE", "tc")
+    ys = [torch.full((T, O), float("nan"), device="cuda") for _ in range(12)]
+    for y in ys:
+        lin.encode(None, x, K, y, O, T)
+    torch.cuda.synchronize()
+    mlxq.streamStatus(None, 0)
+    assert torch.isfinite(ys[0]).all()
+    for y in ys[1:]:
+        assert torch.equal(y, ys[0])
