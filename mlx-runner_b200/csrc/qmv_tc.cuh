@@ -27,7 +27,9 @@
 // those rows, which adds them up in the order of the slices, a block later than it could, so that nobody waits.
 //
 // Two CTAs share an SM: one's waits are the other's turns, and the next launch of the stream can fetch its first stages
-// while this one's last CTAs run.  Every wait but the cluster's start and end is bounded: a wait that runs out sets the
+// while this one's last CTAs run.  (Never three: a CTA asks for 80 KB at the least.  And the library's other kernels that allocate
+// tensor memory fill an SM's registers, so that no two launches wait for each other's.)  Every wait but the cluster's start and end
+// is bounded: a wait that runs out sets the
 // device error word and the CTA's abort flag, and all roles run on to the common exit.
 #pragma once
 
@@ -231,8 +233,8 @@ __device__ __forceinline__ void tc_stage8(uint8_t* xs, int tile_bytes, int part_
 
 // NTK: tokens a drain works for (the batch rounded up); SPLIT: fp16 parts per activation.
 //
-// The code is kept short on purpose: every role's loops are rolled and stand once.  A launch works for 4 to 30 us, and what it
-// runs through only once it waits for, line by line, at the instruction cache.
+// The code is kept short on purpose: every role's loops are rolled and stand once.  A launch on a small layer works for 4 us, and
+// what it runs through only once it waits for, line by line, at the instruction cache.
 template <int BITS, int NTK, int SPLIT>
 __global__ void __launch_bounds__(TC_THREADS, 2)
 qmv_tc_kernel(const __grid_constant__ MmaParams p, const __grid_constant__ TcPlan tp) {
