@@ -138,6 +138,14 @@ def test_tensor_memory_kernel_at_its_edges(mlxq, monkeypatch, call):
     # no single output further off than such a sum can be: six deviations
     worst = ((y[:, :O].double() - ref).abs().max() / ref.pow(2).mean().sqrt()).item()
     assert worst < 6 * bar, f"{worst} of the root mean square"
+    for dtype in (torch.float16, torch.bfloat16):                  # 16-bit outputs: the same sums, rounded once
+        y16 = torch.full((T, O + 3), float("nan"), device="cuda", dtype=dtype)
+        if len(lins) == 1:
+            lins[0].encode(None, x, K + 8, y16, O + 3, T)
+        else:
+            mlxq.Linear.encodeFusedDecode(None, lins, x, y16, K + 8, O + 3, T)
+        torch.cuda.synchronize()
+        assert torch.equal(y16[:, :O], y[:, :O].to(dtype)) and torch.isnan(y16[:, O:]).all()
 
 
 @pytest.mark.parametrize("bits,K,O,T,x_dtype", [(4, 4096, 24576, 6, 0), (4, 4096, 24576, 16, 1), (3, 4096, 11008, 16, 0), (8, 12288, 4096, 8, 0)])
