@@ -374,7 +374,7 @@ static int run_qmv(const mlxq_linear_t* parts, int n, cudaStream_t st, const voi
             }
         }
         if (peer && !rsmem) return fail(MLXQ_UNSUPPORTED, "this shape does not run on the persistent decode kernel: no fused gather");
-        if (const int rc = tensor_memory(fit == 4 ? TcInstead::halves : TcInstead::other); rc >= 0) return rc;
+        if (const int rc = tensor_memory(fit == 4 ? TcInstead::halves : rsmem ? TcInstead::general : TcInstead::other); rc >= 0) return rc;
         if (fit) {
             // ... or two calls of half the tokens: each on a persistent kernel, they beat the register-fed kernel although
             // the weights are read twice.

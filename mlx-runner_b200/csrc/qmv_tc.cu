@@ -21,28 +21,30 @@ int align_up(int v, int a) { return (v + a - 1) / a * a; }
 
 // Whether the kernel is the faster one, by what the call runs on otherwise.  Fitted to 70,000 calls timed on both sides in turn: 6
 // widths, groups of 32, 64 and 128, 33 row counts of 512 ... 151936, 26 row lengths of 512 ... 14336, batches of 2 ... 16 tokens of
-// each type: of the 23,600 calls that the rules take, 0.6 % are more than 1.5 % slower than before, 7 by more than 10 %, and the mean is
-// 2.4 times as fast.  (11008 x 4096, 3 bits, 16 fp32 tokens, in the place of CUDA cores: 361 -> 32 us.)
+// each type: of the 24,100 calls that the rules take, 0.7 % are more than 1.5 % slower than before, 9 by more than 10 %, and the
+// mean is 2.4 times as fast.  (11008 x 4096, 3 bits, 16 fp32 tokens, in the place of CUDA cores: 361 -> 32 us.)
 
 // In the place of one launch of the token-major kernel on single CTAs.  Each of its CTAs stages all of K of the batch: the KB of
-// that decide, less of them where few rows leave it few CTAs to a wave.  us before : with this
-// kernel, groups of 64: 6 fp32 tokens at 4 bits, 4096 x 4096 (96 KB) 12.1 : 10.1, 24576 x 4096 33.5 : 28.7, 24576 x 2048 17.7 : 17.9,
-// 4096 x 1024 5.8 : 6.8; 4 tokens 24576 x 4096 25.9 : 27.3; 6 tokens at 6 bits 151936 x 4096 159 : 175; 8 fp16 tokens at 3 bits
-// 11008 x 4096 (64 KB) 22.5 : 20.3.
+// that decide, fewer of them where there are few rows to share it.  us before : with this kernel, groups of 64: 6 fp32 tokens at
+// 4 bits, 4096 x 4096 (96 KB) 12.1 : 10.1, 24576 x 4096 33.5 : 28.7, 24576 x 2048 17.7 : 17.9, 4096 x 1024 5.8 : 6.8; 4 tokens
+// 24576 x 4096 25.9 : 27.3; 6 tokens at 6 bits 151936 x 4096 159 : 175; 8 fp16 tokens at 3 bits 11008 x 4096 (64 KB) 22.5 : 20.3.
 bool over_token_major(int bits, int gs, int rows, int tokens, int split, int kb) {
     const bool even = bits == 4 || bits == 8, fp32 = split == 2;
     if (gs == 32 && bits == 4 && !fp32) return false;
     if (tokens <= 4) {
         // (few tokens: the other kernel has one set of accumulators and few staged columns)
         if (!fp32) return false;
-        if (tokens == 2) return gs == 64 && bits <= 5 && rows <= 6144 && kb >= 80 && kb <= 96;
+        if (tokens == 2) return gs == 64 && bits <= 5 && rows <= 6144 && (even || bits == 2 ? kb >= 80 && kb <= 96 : kb >= 60);
         if (rows <= 3072) return kb >= (gs == 128 && !even ? 40 : 80);
         if (gs == 32) return bits >= 6 && kb >= (rows <= 15360 ? 72 : 48);
         if (gs == 128 || bits >= 6) return false;
         if (rows <= 15360) return kb >= 80 && (bits != 2 || rows <= 6144);
         return bits != 2 && kb >= (bits == 4 ? 144 : 112);
     }
-    if (gs == 32) return kb >= (rows <= 3072 || bits == 4 || !fp32 || (bits == 6 && rows <= 15360) ? 96 : 56);
+    if (gs == 32) {
+        if (bits == 6 && !fp32 && rows > 15360 && tokens <= 8) return kb >= 56;
+        return kb >= (rows <= 3072 || bits == 4 || !fp32 || (bits == 6 && rows <= 15360) ? 96 : 56);
+    }
     if (gs == 128) {
         if (!even) return rows <= 15360 && kb >= (rows <= 3072 ? 32 : rows <= 6144 ? 40 : 64);
         if (rows <= 3072) return kb >= (bits == 4 ? 56 : 40);
@@ -52,7 +54,7 @@ bool over_token_major(int bits, int gs, int rows, int tokens, int split, int kb)
     if (rows <= 6144) return kb >= (bits == 8 ? 112 : bits == 4 ? 72 : fp32 ? 64 : 56);
     if (fp32) {
         if (rows <= 15360) return kb >= (bits >= 6 ? 112 : bits == 5 ? 80 : 72);
-        return bits >= 3 && bits <= 5 && kb >= (bits == 3 ? 96 : bits == 5 ? 80 : 72);
+        return bits <= 5 && kb >= (bits == 2 ? 144 : bits == 3 ? 96 : bits == 5 ? 80 : 72);
     }
     if (tokens <= 8 && bits >= 3 && bits <= 5) return kb >= (bits == 5 ? 72 : bits == 3 && rows <= 15360 ? 64 : 96);
     return rows <= 15360 && !even && kb >= 112;
@@ -60,17 +62,22 @@ bool over_token_major(int bits, int gs, int rows, int tokens, int split, int kb)
 
 // ... of the token-major kernel with K split over a cluster, `scaled` or not: mostly the taller layers, where its clusters queue
 // (8 fp32 tokens, 4 bits, 11008 x 12288 60.9 : 41.0 us; 6 bits 61.4 : 64.2).
-bool over_cluster(int bits, int gs, int rows, int tokens, int split, bool scaled) {
+bool over_cluster(int bits, int gs, int K, int rows, int tokens, int split, bool scaled) {
     const bool fp32 = split == 2;
-    if (tokens <= 4 || gs == 128) return false;
+    if (tokens <= 4) return false;
+    if (gs != 64 && scaled && fp32 && tokens >= 7 && (bits == 4 || (bits == 2 && gs == 128))) return true;
+    if (gs == 128) return false;
     if (gs == 32) return fp32 && bits >= 6 && rows > 3072;
-    if (!scaled)
-        return fp32 && ((bits == 4 && rows > (tokens >= 6 ? 3072 : 6144)) || (bits == 5 && rows > 6144) || (bits == 3 && rows > 32768));
+    if (!scaled) {
+        if (!fp32) return (bits == 4 || bits == 5) && tokens <= 8 && rows > 6144 && K <= 12288;
+        return (bits == 4 && rows > (tokens >= 6 ? 3072 : 6144)) || (bits == 5 && rows > 6144) || (bits == 3 && rows > 15360);
+    }
     switch (bits) {
-        case 2: return rows <= (fp32 ? 15360 : 3072);
+        case 2: return rows <= (fp32 ? 15360 : 3072) || (fp32 && tokens >= 7);
         case 3: return rows > 6144 && (fp32 || rows <= 15360);
         case 4: return fp32 || rows <= 15360;
         case 5: return rows > 3072;
+        case 8: return fp32 && tokens >= 7 && rows <= 6144 && K <= 12288;
         default: return false;
     }
 }
@@ -79,8 +86,8 @@ bool worth(TcInstead instead, int bits, int gs, int K, int rows, int tokens, int
     switch (instead) {
         case TcInstead::named: return true;
         case TcInstead::token_major: return over_token_major(bits, gs, rows, tokens, split, tokens * split * (K / 128) / 4);      // (K <= STAGED_K_MAX)
-        case TcInstead::cluster: return over_cluster(bits, gs, rows, tokens, split, false);
-        case TcInstead::scaled_cluster: return over_cluster(bits, gs, rows, tokens, split, true);
+        case TcInstead::cluster: return over_cluster(bits, gs, K, rows, tokens, split, false);
+        case TcInstead::scaled_cluster: return over_cluster(bits, gs, K, rows, tokens, split, true);
         case TcInstead::halves:
             // two launches of the token-major kernel, which read the weights twice.  Not where they are near the memory's rate all the
             // same: vocabulary-sized layers, at 8 bits on rows that cut badly (100352 x 2560, 16 fp32 tokens 140 : 205 us), in groups of 128,
@@ -88,7 +95,8 @@ bool worth(TcInstead instead, int bits, int gs, int K, int rows, int tokens, int
             if (rows > 32768 && ((bits == 8 && K > 2048 && K < 4096) || (gs == 128 && K > 3072 && K < 8192))) return false;
             if (rows > 20480 && bits == 6 && K < 1024) return false;
             return true;
-        default: return tokens >= (split == 2 ? 3 : 5);        // kernels on the CUDA cores, or that read the weights several times
+        case TcInstead::general: return tokens >= (split == 2 ? 3 : 5);
+        default: return tokens >= (split == 2 ? 2 : 5);        // kernels on the CUDA cores, or that read the weights several times
     }
 }
 

@@ -634,8 +634,9 @@ struct TcRoom {
 };
 const TcRoom& qmv_tc_room(int device, int sms);
 
-// What a call runs on where the kernel does not take it: `named` is a call that the kernel takes whenever it can serve it.
-enum class TcInstead { named, token_major, cluster, scaled_cluster, halves, other };
+// What a call runs on where the kernel does not take it (`general`: the one-token kernel's general plan); `named` is a call that the
+// kernel takes whenever it can serve it.
+enum class TcInstead { named, token_major, cluster, scaled_cluster, halves, general, other };
 
 // Plans a call; returns the shared memory it needs, 0 when the call is not one the kernel serves, or not one that it is the faster
 // for than what the call runs on otherwise.

@@ -12,7 +12,7 @@ ROOT = os.path.dirname(HERE)
 PKG = os.path.join(ROOT, "mlx-runner_b200")
 
 SMEM_OPT_IN = 227 * 1024
-NAMED, TOKEN_MAJOR, CLUSTER, SCALED_CLUSTER, HALVES, OTHER = range(6)       # enum TcInstead
+NAMED, TOKEN_MAJOR, CLUSTER, SCALED_CLUSTER, HALVES, GENERAL, OTHER = range(7)       # enum TcInstead
 
 
 @pytest.fixture(scope="module")
@@ -88,8 +88,8 @@ def test_clusters_are_the_ones_that_the_device_holds(plans):
     ((8, 64, 4096, 3072, 6, 2), TOKEN_MAJOR, True), ((8, 64, 4096, 3080, 6, 2), TOKEN_MAJOR, False),
     # two launches of half the tokens; not vocabulary-sized layers at 8 bits on rows that cut badly
     ((8, 64, 2560, 32768, 16, 2), HALVES, True), ((8, 64, 2560, 32776, 16, 2), HALVES, False), ((4, 64, 2560, 151936, 16, 2), HALVES, True),
-    # in the place of kernels without tensor cores, from three fp32 or five 16-bit tokens on
-    ((2, 32, 512, 4096, 3, 2), OTHER, True), ((2, 32, 512, 4096, 2, 2), OTHER, False), ((2, 32, 512, 4096, 5, 1), OTHER, True), ((2, 32, 512, 4096, 4, 1), OTHER, False),
+    # in the place of kernels without tensor cores, from two fp32 (three, of the general plan) or five 16-bit tokens on
+    ((2, 32, 512, 4096, 2, 2), OTHER, True), ((2, 32, 512, 4096, 3, 2), GENERAL, True), ((2, 32, 512, 4096, 2, 2), GENERAL, False), ((2, 32, 512, 4096, 5, 1), OTHER, True), ((2, 32, 512, 4096, 4, 1), OTHER, False),
     # 8 bits with 16-bit activations: while the sums are short enough
     ((8, 32, 8192, 4096, 16, 1), OTHER, True), ((8, 32, 12288, 4096, 16, 1), OTHER, False), ((8, 64, 14336, 4096, 16, 1), OTHER, True),
     # what the kernel cannot serve
